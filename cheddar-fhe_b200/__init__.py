@@ -1,4 +1,5 @@
-"""Python binding of libcheddar_b200.so through its C ABI (ctypes).
+"""Python binding of libcheddar_b200.so through its C ABI: the per-operation
+calls through a CPython module (host/py_calls.c), set-up calls through ctypes.
 
 The directory name carries a hyphen, so load it with
 `importlib.util.spec_from_file_location("cheddar_fhe_b200", ".../__init__.py")`
@@ -7,6 +8,7 @@ only for device memory and streams; every operation goes through the shared
 library, and a missing library is an error, never a fallback.
 """
 import ctypes as C
+import importlib.util
 import json
 import os
 import subprocess
@@ -17,10 +19,12 @@ from . import client  # noqa: F401  (host-side keygen / encrypt / encode)
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "lib", "libcheddar_b200.so")
+CALLS_PATH = os.path.join(_HERE, "lib", "cheddar_b200_calls.so")
 HEADER_PATH = os.path.join(os.path.dirname(_HERE), "include", "cheddar_b200.h")
 PARAM_DIR = os.path.join(_HERE, "parameters")
 
 _lib = None
+_calls = None
 
 
 def build(verbose=False):
@@ -40,9 +44,26 @@ def lib():
         L = C.CDLL(LIB_PATH)
         L.cfhe_last_error.restype = C.c_char_p
         L.cfhe_prime.restype = C.c_uint32
+        L.cfhe_galois_for_rotation.restype = C.c_uint32
         L.cfhe_kernel_launch_count.restype = C.c_ulonglong
         _lib = L
     return _lib
+
+
+def calls():
+    """The module of host/py_calls.c."""
+    global _calls
+    if _calls is None:
+        lib()
+        if not os.path.exists(CALLS_PATH):
+            raise RuntimeError(
+                f"{CALLS_PATH} is missing: build it with `make -C {_HERE}`; there is no fallback path")
+        spec = importlib.util.spec_from_file_location("cheddar_b200_calls", CALLS_PATH)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        mod.set_converters(lambda a: _ints(a)[0], lambda a: _u32s(a)[0])
+        _calls = mod
+    return _calls
 
 
 def kernel_launch_count():
@@ -86,6 +107,7 @@ class Engine:
 
         self.torch = torch
         self.L = lib()
+        self.K = calls()
         self.p = params
         self.device = device
         main, mp = _u32s(params["main_primes"])
@@ -98,6 +120,7 @@ class Engine:
             tp, len(params["terminal_primes"]), ap, len(params["auxiliary_primes"]),
             lp, len(params["level_config"]), params["additional_base"][0], params["additional_base"][1]))
         self.h = h
+        self.hp = h.value  # the handle as the calls of self.K take it
         self.n = self.L.cfhe_degree(h)
         self.num_primes = self.L.cfhe_num_primes(h)
         self.primes = np.array([self.L.cfhe_prime(h, g) for g in range(self.num_primes)], dtype=np.uint64)
@@ -109,6 +132,7 @@ class Engine:
         if getattr(self, "h", None):
             self.L.cfhe_context_destroy(self.h)
             self.h = None
+            self.hp = 0
 
     def __del__(self):
         try:
@@ -156,25 +180,10 @@ class Engine:
 
     # ---- device-resident API: tensors [polys, limbs, N] or [limbs, N]
     def ntt_(self, dst, src, gidx, mont_conv=False):
-        g, gp = _ints(gidx)
-        polys = 1 if src.dim() == 2 else src.shape[0]
-        stride_s = src.stride(0) if src.dim() == 3 else 0
-        stride_d = dst.stride(0) if dst.dim() == 3 else 0
-        self._check(self.L.cfhe_ntt(self.h, self._p(dst), self._p(src), gp, len(g), polys,
-                                    C.c_longlong(stride_d), C.c_longlong(stride_s), int(mont_conv)))
+        self._check(self.K.ntt(self.hp, dst, src, gidx, mont_conv))
 
     def intt_(self, dst, src, gidx, consts=None, mont_keep=False, centred=False):
-        g, gp = _ints(gidx)
-        polys = 1 if src.dim() == 2 else src.shape[0]
-        stride_s = src.stride(0) if src.dim() == 3 else 0
-        stride_d = dst.stride(0) if dst.dim() == 3 else 0
-        if consts is not None:
-            k, kp = _u32s(consts)
-        else:
-            kp = None
-        self._check(self.L.cfhe_intt(self.h, self._p(dst), self._p(src), gp, len(g), polys,
-                                     C.c_longlong(stride_d), C.c_longlong(stride_s), kp,
-                                     int(mont_keep), int(centred)))
+        self._check(self.K.intt(self.hp, dst, src, gidx, consts, mont_keep, centred))
 
     # ---- host-array API with the golden model's signatures (copies in/out)
     def ntt(self, src, gidx, mont_conv=False):
@@ -203,7 +212,6 @@ class Engine:
         return self._check(self.L.cfhe_beta(self.h, level))
 
     def galois(self, rot):
-        self.L.cfhe_galois_for_rotation.restype = C.c_uint32
         return self.L.cfhe_galois_for_rotation(self.h, int(rot))
 
     def _alpha(self, level):
@@ -215,30 +223,17 @@ class Engine:
 
     # ---- device-resident operators
     def binary_(self, op, dst, a, b, gidx):
-        g, gp = _ints(gidx)
-        self._check(self.L.cfhe_binary(self.h, op, self._p(dst), self._p(a),
-                                       self._p(b) if b is not None else None, gp, len(g)))
+        self._check(self.K.binary(self.hp, op, dst, a, b, gidx))
 
     def const_op_(self, op, dst, a, b, consts, gidx):
-        g, gp = _ints(gidx)
-        k, kp = _u32s(consts)
-        self._check(self.L.cfhe_const_op(self.h, op, self._p(dst), self._p(a),
-                                         self._p(b) if b is not None else None, kp, gp, len(g)))
+        self._check(self.K.const_op(self.hp, op, dst, a, b, consts, gidx))
 
     def elementwise_multi_(self, with_const, op, dsts, a_list, b_list, consts, gidx):
         """One launch for several polynomials (cfhe_elementwise_multi)."""
-        g, gp = _ints(gidx)
-        n = len(dsts)
-        arr = lambda ts: (C.c_void_p * n)(*[t.data_ptr() if t is not None else None for t in ts])
-        kp = None
-        if consts is not None:
-            k, kp = _u32s(consts)
-        self._check(self.L.cfhe_elementwise_multi(self.h, int(with_const), int(op), n, arr(dsts), arr(a_list),
-                                                  arr(b_list) if b_list is not None else None, kp, gp, len(g)))
+        self._check(self.K.elementwise_multi(self.hp, with_const, op, dsts, a_list, b_list, consts, gidx))
 
     def tensor_(self, d0, d1, d2, b1, a1, b2, a2, gidx):
-        g, gp = _ints(gidx)
-        self._check(self.L.cfhe_tensor(self.h, *[self._p(t) for t in (d0, d1, d2, b1, a1, b2, a2)], gp, len(g)))
+        self._check(self.K.tensor(self.hp, d0, d1, d2, b1, a1, b2, a2, gidx))
 
     def tensor_accum_(self, d0, d1, d2, b1s, a1s, b2s, a2s, gidx, accumulate=False):
         """(d0, d1, d2) (+)= sum_t tensor(b1s[t], a1s[t], b2s[t], a2s[t]) (cfhe_tensor_accum)."""
@@ -258,10 +253,7 @@ class Engine:
                                                  gp, len(g)))
 
     def permute_(self, dst, src, add, galois, gidx):
-        g, gp = _ints(gidx)
-        self._check(self.L.cfhe_permute(self.h, self._p(dst), self._p(src),
-                                        self._p(add) if add is not None else None,
-                                        C.c_uint32(int(galois)), gp, len(g)))
+        self._check(self.K.permute(self.hp, dst, src, add, galois, gidx))
 
     def nary_(self, kind, dsts, terms, gidx, consts=None, pts=None, galois=None, addend=None):
         """Fused n-ary sums (cfhe_accum / cfhe_caccum / cfhe_paccum /
@@ -301,19 +293,13 @@ class Engine:
 
     def ctpt_gemm_(self, ys, xs, packed, gidx):
         """ys[j] = sum_k W[k][j] * xs[k] on the tensor cores (cfhe_ctpt_gemm)."""
-        g, gp = _ints(gidx)
-        self._check(self.L.cfhe_ctpt_gemm(self.h, self._ptrs(ys), self._ptrs(xs), C.c_void_p(packed.data_ptr()),
-                                          len(xs), len(ys), gp, len(g)))
+        self._check(self.K.ctpt_gemm(self.hp, ys, xs, packed, gidx))
 
     def sample_uniform_(self, dst, gidx, seed, stream=0):
-        g, gp = _ints(gidx)
-        self._check(self.L.cfhe_sample_uniform(self.h, self._p(dst), gp, len(g), C.c_ulonglong(seed),
-                                               C.c_uint(stream)))
+        self._check(self.K.sample_uniform(self.hp, dst, gidx, seed, stream))
 
     def sample_error_(self, dst, gidx, sigma, seed, stream=0):
-        g, gp = _ints(gidx)
-        self._check(self.L.cfhe_sample_error(self.h, self._p(dst), gp, len(g), C.c_double(sigma),
-                                             C.c_ulonglong(seed), C.c_uint(stream)))
+        self._check(self.K.sample_error(self.hp, dst, gidx, sigma, seed, stream))
 
     def error_cdf(self, sigma):
         out = np.zeros(97, dtype=np.uint64)
@@ -321,17 +307,14 @@ class Engine:
         return out
 
     def encrypt_(self, b, a, s, e, m, gidx):
-        g, gp = _ints(gidx)
-        self._check(self.L.cfhe_encrypt(self.h, self._p(b), self._p(a), self._p(s), self._p(e),
-                                        self._p(m) if m is not None else None, gp, len(g)))
+        self._check(self.K.encrypt(self.hp, b, a, s, e, m, gidx))
 
     def encode_coeffs_(self, dst, coeffs, gidx):
         """dst = NTT (M-form) of the residues of trunc(coeffs[i]) on the limbs of gidx
         (cfhe_encode_coeffs); coeffs: N float64 values on the host."""
-        g, gp = _ints(gidx)
         c = np.ascontiguousarray(coeffs, dtype=np.float64)
         assert c.shape == (self.n,)
-        self._check(self.L.cfhe_encode_coeffs(self.h, self._p(dst), c.ctypes.data_as(C.c_void_p), gp, len(g)))
+        self._check(self.K.encode_coeffs(self.hp, dst, c, gidx))
 
     def add_evk_part_(self, bx, s_target, p_prod, gidx):
         g, gp = _ints(gidx)
@@ -346,11 +329,7 @@ class Engine:
 
     def moddown_(self, level, kind, dst, src):
         """dst/src: [limbs, N] or [polys, limbs, N]."""
-        polys = 1 if src.dim() == 2 else src.shape[0]
-        ss = src.stride(0) if src.dim() == 3 else 0
-        ds = dst.stride(0) if dst.dim() == 3 else 0
-        self._check(self.L.cfhe_moddown(self.h, level, kind, self._p(dst), self._p(src), polys,
-                                        C.c_longlong(ds), C.c_longlong(ss)))
+        self._check(self.K.moddown(self.hp, level, kind, dst, src))
 
     def moddown_staged_(self, level, kind, dst, src):
         """The same as moddown_, composed from the three stage entries
@@ -380,18 +359,11 @@ class Engine:
                                           self._ptrs(evk_b), self._ptrs(evk_a), int(key_main)))
 
     def keyswitch_(self, level, out_b, out_a, d, bx, evk_b, evk_a, key_main):
-        self._check(self.L.cfhe_keyswitch(self.h, level, self._p(out_b), self._p(out_a), self._p(d),
-                                          self._p(bx) if bx is not None else None,
-                                          self._ptrs(evk_b), self._ptrs(evk_a), int(key_main)))
+        self._check(self.K.keyswitch(self.hp, level, out_b, out_a, d, bx, evk_b, evk_a, key_main))
 
     def hoisted_rotations_(self, level, out, bx, ax, rots, evk_b, evk_a, key_main):
         """out: [n_rot, 2, nq, N]; evk_b/evk_a: per rotation a list of beta digit tensors."""
-        r, rp = _ints(rots)
-        flat_b = [t for key in evk_b for t in key]
-        flat_a = [t for key in evk_a for t in key]
-        self._check(self.L.cfhe_hoisted_rotations(self.h, level, self._p(out), self._p(bx), self._p(ax),
-                                                  len(r), rp, self._ptrs(flat_b), self._ptrs(flat_a),
-                                                  int(key_main)))
+        self._check(self.K.hoisted_rotations(self.hp, level, out, bx, ax, rots, evk_b, evk_a, key_main))
 
     def linear_transform_(self, level, out_b, out_a, in_b, in_a, baby_rots, baby_keys, giant_rots,
                           giant_keys, pts, key_main, rescale=True):
@@ -399,22 +371,8 @@ class Engine:
         baby_rots[0] must be 0. baby_keys / giant_keys: per step a pair
         (digits_b, digits_a) of lists of beta device tensors, or None for an
         unrotated step. pts[j][i]: device tensor [(nq+alpha), N] or None."""
-        beta = self.beta(level)
-
-        def flat(keys, part):
-            out = []
-            for k in keys:
-                out += [None] * beta if k is None else list(k[part][:beta])
-            return (C.c_void_p * len(out))(*[t.data_ptr() if t is not None else None for t in out])
-
-        br, brp = _ints(baby_rots)
-        gr, grp = _ints(giant_rots)
-        ptl = [pts[j][i] for j in range(len(gr)) for i in range(len(br))]
-        pta = (C.c_void_p * len(ptl))(*[t.data_ptr() if t is not None else None for t in ptl])
-        self._check(self.L.cfhe_linear_transform(
-            self.h, level, int(rescale), self._p(out_b), self._p(out_a), self._p(in_b), self._p(in_a),
-            len(br), brp, flat(baby_keys, 0), flat(baby_keys, 1),
-            len(gr), grp, flat(giant_keys, 0), flat(giant_keys, 1), pta, int(key_main)))
+        self._check(self.K.linear_transform(self.hp, level, out_b, out_a, in_b, in_a, baby_rots, baby_keys,
+                                            giant_rots, giant_keys, pts, key_main, rescale))
 
     def modup_to_max_(self, dst, src, src_gidx, dst_gidx):
         """Exact centred lift of a one- or two-limb value (cfhe_modup_to_max)."""
@@ -428,9 +386,7 @@ class Engine:
         return self.to_host(d)
 
     def hmult_(self, level, out_b, out_a, b1, a1, b2, a2, evk_b, evk_a, key_main, rescale=True):
-        self._check(self.L.cfhe_hmult(self.h, level, self._p(out_b), self._p(out_a),
-                                      self._p(b1), self._p(a1), self._p(b2), self._p(a2),
-                                      self._ptrs(evk_b), self._ptrs(evk_a), int(key_main), int(rescale)))
+        self._check(self.K.hmult(self.hp, level, out_b, out_a, b1, a1, b2, a2, evk_b, evk_a, key_main, rescale))
 
     # ---- host-array operators with the golden model's signatures
     def _bin(self, op, a, b, gidx):
