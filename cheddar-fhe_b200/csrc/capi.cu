@@ -164,6 +164,16 @@ int cfhe_context_create(cfhe_context **out, int device, int log_degree,
     e = cudaMemcpy(c.d_tw, fwd.data(), tsz * sizeof(Tw), cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
     e = cudaMemcpy(c.d_itw, inv.data(), tsz * sizeof(Tw), cudaMemcpyHostToDevice);
+  {
+    std::vector<Tw> rows(tsz);
+    for (int dir = 0; dir < 2 && e == cudaSuccess; dir++) {
+      uint4 **d = dir ? &c.d_row_itw : &c.d_row_tw;
+      for (int g = 0; g < c.NP; g++)
+        build_row_twiddles((dir ? inv : fwd).data() + (size_t)g * c.n, c.logn, rows.data() + (size_t)g * c.n);
+      e = cudaMalloc(d, tsz * sizeof(Tw));
+      if (e == cudaSuccess) e = cudaMemcpy(*d, rows.data(), tsz * sizeof(Tw), cudaMemcpyHostToDevice);
+    }
+  }
   if (e != cudaSuccess) return cleanup_fail(cudaGetErrorString(e));
   if (build_plans(c) != 0 || noalloc_prepare(device) != 0) {
     std::string m = get_error();
@@ -184,6 +194,8 @@ void cfhe_context_destroy(cfhe_context *h) {
   free_plans(c);
   if (c.d_tw) cudaFree(c.d_tw);
   if (c.d_itw) cudaFree(c.d_itw);
+  if (c.d_row_tw) cudaFree(c.d_row_tw);
+  if (c.d_row_itw) cudaFree(c.d_row_itw);
   if (c.own_stream && c.stream) cudaStreamDestroy(c.stream);
   delete h;
 }

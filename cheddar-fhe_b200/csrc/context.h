@@ -94,6 +94,10 @@ struct Context {
   std::vector<uint32_t> psi;  // primitive 2N-th roots in that order
 
   Tw *d_tw = nullptr, *d_itw = nullptr;  // [NP][N]
+  // Twiddles of the four stages inside blocks of 16 words, in the order the
+  // threads of a row read them: [NP][row][8][16] chunks of two (the 16th of a
+  // thread is padding)
+  uint4 *d_row_tw = nullptr, *d_row_itw = nullptr;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
 

@@ -86,4 +86,21 @@ inline void build_twiddles(uint32_t q, int logn, Tw *fwd, Tw *inv,
   for (int j = 0; j < n; j++) inv[j] = make_tw(pw[bitrev(j, logn)], q);
 }
 
+// The entries of a forward or inverse table that the four stages inside blocks
+// of 16 words use, in reading order: for row R and thread t of the row, pairs
+// {0,1}, {2,3}, ... of the 15 twiddles (one of stage 0, two of stage 1, ...)
+// at out[2 * (R * 128 + pair * 16 + t)]. In table order the threads of a row
+// read the last stage's twiddles 64 bytes apart.
+inline void build_row_twiddles(const Tw *table, int logn, Tw *out) {
+  const int rows = (1 << logn) >> 8;
+  for (int R = 0; R < rows; R++)
+    for (int t = 0; t < 16; t++) {
+      const int i0 = (1 << (logn - 4)) + 16 * R + t;
+      int k = 0;
+      for (int s = 0; s < 4; s++)
+        for (int e = 0; e < 1 << s; e++, k++) out[2 * (R * 128 + (k / 2) * 16 + t) + (k & 1)] = table[(i0 << s) + e];
+      out[2 * (R * 128 + 7 * 16 + t) + 1] = Tw{0, 0};
+    }
+}
+
 }  // namespace cfhe
