@@ -77,16 +77,19 @@ struct TensorAccArgs {
 };
 
 constexpr int kMaxDigits = 8;
+// Key inner products of one decomposition with up to kMaxInnerRots keys; the
+// results of key r lie r * 2 * ntot limbs after acc_b / acc_a.
+constexpr int kMaxInnerRots = 4;
 struct InnerArgs {
   uint32_t *acc_b, *acc_a;
   const uint32_t *mu;  // ModUp buffers, slot s at mu + s*ntot*N
   const uint32_t *d;   // polynomial being switched (own limbs), or null
   const uint32_t *c0, *c1;  // optional P*c0 -> acc_b, P*c1 -> acc_a (Q limbs)
-  const uint32_t *kb[kMaxDigits], *ka[kMaxDigits];
-  int n_digits, ntot, nq;
+  const uint32_t *kb[kMaxInnerRots][kMaxDigits], *ka[kMaxInnerRots][kMaxDigits];
+  int n_rots, n_digits, ntot, nq;
   // 0: results stay in place; otherwise the inverse Galois element g^-1 of an
   // automorphism applied to the result: word i is stored at pi_{g^-1}(i)
-  uint32_t scatter_galois;
+  uint32_t scatter_galois[kMaxInnerRots];
   int accumulate;  // != 0: the result is added to what acc_b / acc_a hold
   uint8_t mu_slot[kMaxDigits];
   uint32_t q[kMaxLimbs], nqinv[kMaxLimbs], pm[kMaxLimbs];
@@ -121,7 +124,7 @@ struct BconvTcJob {
 };
 struct BconvTcArgs {
   int n_jobs;
-  int per_unit;     // CTAs sharing the tiles of one job (filled by the launcher)
+  int per_unit;     // CTAs sharing the tiles of one unit (filled by the launcher)
   int *error_flag;  // set to 1 when a completion wait timed out
   BconvTcJob jobs[kMaxBconvJobs];
 };

@@ -247,33 +247,14 @@ int run_moddown(const Context &c, const ConvPlan &cv, uint32_t *dst,
   return run_moddown_ntt(c, cv, dst, src, n_polys, dst_stride, src_stride);
 }
 
+// One key per entry of `galois_inv` (n_rots of them, 0: no automorphism); the
+// keys of entry r are kb + r * lp.beta, its results 2 * ntot limbs further on.
 static int run_inner_impl(const Context &c, const LevelPlan &lp, uint32_t *acc_b,
                           uint32_t *acc_a, const uint32_t *mu, const uint32_t *d,
                           const uint32_t *c0, const uint32_t *c1,
                           const uint32_t *const *kb, const uint32_t *const *ka,
-                          int key_main, uint32_t galois_inv, bool accumulate = false);
-
-int run_inner(const Context &c, const LevelPlan &lp, uint32_t *acc_b,
-              uint32_t *acc_a, const uint32_t *mu, const uint32_t *d,
-              const uint32_t *c0, const uint32_t *c1,
-              const uint32_t *const *kb, const uint32_t *const *ka,
-              int key_main) {
-  return run_inner_impl(c, lp, acc_b, acc_a, mu, d, c0, c1, kb, ka, key_main, 0);
-}
-
-int run_inner_rot(const Context &c, const LevelPlan &lp, uint32_t *acc_b,
-                  uint32_t *acc_a, const uint32_t *mu, const uint32_t *d,
-                  const uint32_t *c0, const uint32_t *const *kb,
-                  const uint32_t *const *ka, int key_main, uint32_t galois_inv) {
-  return run_inner_impl(c, lp, acc_b, acc_a, mu, d, c0, nullptr, kb, ka, key_main, galois_inv);
-}
-
-static int run_inner_impl(const Context &c, const LevelPlan &lp, uint32_t *acc_b,
-                          uint32_t *acc_a, const uint32_t *mu, const uint32_t *d,
-                          const uint32_t *c0, const uint32_t *c1,
-                          const uint32_t *const *kb, const uint32_t *const *ka,
-                          int key_main, uint32_t galois_inv, bool accumulate) {
-  if ((int)lp.digits.size() > kMaxDigits) {
+                          int key_main, int n_rots, const uint32_t *galois_inv, bool accumulate = false) {
+  if ((int)lp.digits.size() > kMaxDigits || n_rots > kMaxInnerRots) {
     set_error("inner product: too many digits");
     return -1;
   }
@@ -290,15 +271,18 @@ static int run_inner_impl(const Context &c, const LevelPlan &lp, uint32_t *acc_b
   a.d = d;
   a.c0 = c0;
   a.c1 = c1;
+  a.n_rots = n_rots;
   a.n_digits = (int)lp.digits.size();
   a.ntot = lp.ntot;
   a.nq = lp.nq;
-  a.scatter_galois = galois_inv;
   a.accumulate = accumulate ? 1 : 0;
+  for (int r = 0; r < n_rots; r++) a.scatter_galois[r] = galois_inv[r];
   for (int i = 0; i < a.n_digits; i++) {
     const int slot = lp.digits[i].index;
-    a.kb[i] = kb[slot];
-    a.ka[i] = ka[slot];
+    for (int r = 0; r < n_rots; r++) {
+      a.kb[r][i] = kb[(size_t)r * lp.beta + slot];
+      a.ka[r][i] = ka[(size_t)r * lp.beta + slot];
+    }
     a.mu_slot[i] = (uint8_t)slot;
   }
   for (int l = 0; l < lp.ntot; l++) {
@@ -313,6 +297,22 @@ static int run_inner_impl(const Context &c, const LevelPlan &lp, uint32_t *acc_b
   if (int r = launch_inner(c, a)) return r;
   c.mark("inner");
   return 0;
+}
+
+int run_inner(const Context &c, const LevelPlan &lp, uint32_t *acc_b,
+              uint32_t *acc_a, const uint32_t *mu, const uint32_t *d,
+              const uint32_t *c0, const uint32_t *c1,
+              const uint32_t *const *kb, const uint32_t *const *ka,
+              int key_main) {
+  const uint32_t none = 0;
+  return run_inner_impl(c, lp, acc_b, acc_a, mu, d, c0, c1, kb, ka, key_main, 1, &none);
+}
+
+int run_inner_rot(const Context &c, const LevelPlan &lp, uint32_t *acc_b,
+                  uint32_t *acc_a, const uint32_t *mu, const uint32_t *d,
+                  const uint32_t *c0, const uint32_t *const *kb,
+                  const uint32_t *const *ka, int key_main, uint32_t galois_inv) {
+  return run_inner_impl(c, lp, acc_b, acc_a, mu, d, c0, nullptr, kb, ka, key_main, 1, &galois_inv);
 }
 
 int run_tensor(const Context &c, const LevelPlan &lp, uint32_t *d0,
@@ -364,7 +364,7 @@ static uint32_t galois_inverse(uint32_t g) {
   return inv;
 }
 
-constexpr int kHoistChunk = 4;  // rotations whose ModDowns share launches
+constexpr int kHoistChunk = kMaxInnerRots;  // rotations that share an inner product and ModDown launches
 
 size_t hoisted_scratch_words(const LevelPlan &lp) {
   const size_t y_words = std::max(modup_scratch_words(lp),
@@ -389,19 +389,18 @@ int run_hoisted_rotations(Context &c, const LevelPlan &lp, uint32_t *out,
   if (int r = run_modup(c, lp, mu, a, false, y)) return r;
   for (int r0 = 0; r0 < n_rot; r0 += kHoistChunk) {
     const int cnt = std::min(kHoistChunk, n_rot - r0);
+    uint32_t inv[kHoistChunk];
     for (int i = 0; i < cnt; i++) {
       const uint32_t g = galois[r0 + i];
       if ((g & 1u) == 0 || g >= m2) {
         set_error("hoisted rotations: invalid Galois element");
         return -1;
       }
-      const uint32_t inv = galois_inverse(g);
-      uint32_t *ab = acc + (size_t)(2 * i) * acc_words;
-      if (int rc = run_inner_rot(c, lp, ab, ab + acc_words, mu, a, b,
-                                 kb + (size_t)(r0 + i) * lp.beta,
-                                 ka + (size_t)(r0 + i) * lp.beta, key_main, inv))
-        return rc;
+      inv[i] = galois_inverse(g);
     }
+    if (int rc = run_inner_impl(c, lp, acc, acc + acc_words, mu, a, b, nullptr, kb + (size_t)r0 * lp.beta,
+                                ka + (size_t)r0 * lp.beta, key_main, cnt, inv))
+      return rc;
     if (int rc = run_moddown(c, cv, out + (size_t)(2 * r0) * out_words, acc, 2 * cnt,
                              (long long)out_words, (long long)acc_words, y))
       return rc;
@@ -569,9 +568,10 @@ int run_linear_transform(Context &c, const LevelPlan &lp, bool rescale, uint32_t
     }
     for (int i = 1; i < n_baby; i++) {
       uint32_t *rb = rot + (size_t)(2 * i) * ext;
+      const uint32_t inv = galois_inverse(baby_galois[i]);
       if (int r = run_inner_impl(c, lp, rb, rb + ext, mu, in_a, in_b, nullptr,
                                  baby_kb + (size_t)i * lp.beta, baby_ka + (size_t)i * lp.beta,
-                                 key_main, galois_inverse(baby_galois[i])))
+                                 key_main, 1, &inv))
         return r;
     }
     PtAccumArgs pa;
@@ -622,9 +622,10 @@ int run_linear_transform(Context &c, const LevelPlan &lp, bool rescale, uint32_t
     }
     const uint32_t *ca = cj + (size_t)jj * qw;
     if (int r = run_modup(c, lp, mu, ca, false, y)) return r;
+    const uint32_t inv = galois_inverse(g);
     if (int r = run_inner_impl(c, lp, total, total + ext, mu, ca, nullptr, nullptr,
                                giant_kb + (size_t)j * lp.beta, giant_ka + (size_t)j * lp.beta,
-                               key_main, galois_inverse(g), true))
+                               key_main, 1, &inv, true))
       return r;
   }
   // 5. one ModDown (with the rescale) for the whole transform

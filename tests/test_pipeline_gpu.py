@@ -386,3 +386,23 @@ def test_limb_sharded_hmult_on_one_rank_equals_hmult(engine40, params40):
                                            [e.to_dev(ka[i][rows]) for i in active])
         want_b, want_a = e.hmult(level, *ins, kb, ka, M, False)
         assert np.array_equal(e.to_host(got_b), want_b) and np.array_equal(e.to_host(got_a), want_a), level
+
+
+@pytest.mark.parametrize("level", [1, 7, 14, 20, 28])
+@pytest.mark.parametrize("count", [2, 3, 4, 5])
+def test_rotations_sharing_a_launch_equal_single_ones(engine40, level, count):
+    """Two to four rotations share one inner-product launch (a kernel per number
+    of digits); a call with one rotation takes the single-key kernel."""
+    e = engine40
+    rng = np.random.default_rng(7000 + 10 * level + count)
+    g, beta = e.level_limbs(level), e.beta(level)
+    bx, ax = (e.to_dev(rand_limbs(rng, e.primes, g, e.n)) for _ in range(2))
+    rots = [1, 32767, 4096, -3, 77][:count]
+    keys = [fake_key(rng, e, e, 43, beta) for _ in range(2)]
+    dk = [([e.to_dev(x) for x in kb], [e.to_dev(x) for x in ka]) for kb, ka in keys]
+    dk = [dk[i % 2] for i in range(count)]
+    out, one = e.empty(count, 2, len(g), e.n), e.empty(1, 2, len(g), e.n)
+    e.hoisted_rotations_(level, out, bx, ax, rots, [k[0] for k in dk], [k[1] for k in dk], 43)
+    for i, r in enumerate(rots):
+        e.hoisted_rotations_(level, one, bx, ax, [r], [dk[i][0]], [dk[i][1]], 43)
+        assert e.torch.equal(out[i], one[0]), r
