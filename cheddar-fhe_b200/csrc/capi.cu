@@ -499,6 +499,7 @@ int cfhe_intt(cfhe_context *h, uint32_t *dst, const uint32_t *src,
       k = mont_keep ? ninv : mulmod(ninv, rinv_mod(q), q);
     }
     a.kc[l] = make_tw(k, q);
+    a.kcw[l] = make_tw(mulmod(k, c.inv_w1[a.g[l]], q), q);
   }
   { int r_ = launch_ntt(c, a, true); c.mark("intt"); return r_; }
 }

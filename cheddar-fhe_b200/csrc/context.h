@@ -42,6 +42,7 @@ struct NttArgs {
   uint16_t dst_limb[kMaxJobs];
   uint32_t q[kMaxJobs];
   Tw kc[kMaxLimbs];  // per-limb constant (Shoup pair)
+  Tw kcw[kMaxLimbs];  // inverse: the same times the last stage's twiddle
   uint8_t ep_limb[kMaxLimbs];
   Tw ep_pad[kMaxLimbs], ep_scale[kMaxLimbs];
   Tw ep_ps[kMaxLimbs];  // pad * scale, so that the epilogue is pad*scale*x - scale*ntt
@@ -62,6 +63,7 @@ struct ConvPlan {
   bool has_pad = false;
   // the same constants as Shoup pairs, ready for the kernels' argument blocks
   std::vector<Tw> pre_tw;           // pre * 2^-32 (the inverse transform's per-limb constant)
+  std::vector<Tw> pre_w1_tw;        // pre_tw * the twiddle of the inverse transform's last stage
   std::vector<Tw> ep_pad_tw, ep_scale_tw, ep_ps_tw;  // ep_ps = ep_pad * ep_scale
 };
 
@@ -106,11 +108,6 @@ struct Context {
   bool use_fused_lt = true;         // baby steps and plaintext accumulation in one kernel (CFHE_LT=unfused disables)
   bool use_pdl = true;              // programmatic dependent launch between the kernels of a stream (CFHE_PDL=0 disables)
   bool use_twopass_ntt = true;      // two-pass NTT meeting in L2 (CFHE_NTT=cluster selects the cluster kernels)
-  // Pipelined NTT (ntt_tiled.cu): 0 never, 1 when the call batches enough limb
-  // transforms per prime to amortise its set-up (the default), 2 always
-  int ntt_policy = 1;
-  int ntt_chunk = 0;                // limb transforms per launch pair, so that the passes meet in L2 (CFHE_NTT_CHUNK)
-  int ntt_unit = 0;                 // limb transforms of one prime per CTA (CFHE_NTT_UNIT)
   std::vector<uint32_t> inv_w1;     // per prime: entry 1 of the inverse twiddle table (the last inverse stage's twiddle)
   int *d_error_flag = nullptr;      // raised by a kernel whose bounded wait ran out
   cudaEvent_t order_event = nullptr;  // recorded by cfhe_order_after when this context is the earlier one
@@ -226,7 +223,5 @@ inline cudaError_t launch_kernel(bool pdl, void (*kernel)(KArgs...), dim3 grid, 
 
 int launch_ntt(const Context &ctx, const NttArgs &args, bool inverse);
 int launch_ntt_twopass(const Context &ctx, const NttArgs &args, bool inverse);
-int launch_ntt_tiled(const Context &ctx, const NttArgs &args, bool inverse);
-bool ntt_tiled_usable(const Context &ctx, const NttArgs &args);
 
 }  // namespace cfhe

@@ -257,6 +257,35 @@ CFHE_HD void gs_radix16_pre(uint32_t *v, const Tw *t, uint32_t q, uint32_t q2) {
   for (int e = 0; e < 8; e++) gs_bfly<FAST>(v[e], v[e + 8], t[0], q, q2);
 }
 
+// gs_radix16_pre as the last phase of the inverse transform: the last stage's
+// sums are multiplied by kc and its differences by kcw = kc * t[0], so that
+// the per-limb constant costs one product for half of the words only and the
+// sums need no fold. Values below 2q.
+template <bool FAST>
+CFHE_HD void gs_radix16_last(uint32_t *v, const Tw *t, Tw kc, Tw kcw, uint32_t q, uint32_t q2) {
+#pragma unroll
+  for (int j = 0; j < 8; j++) gs_bfly<FAST>(v[2 * j], v[2 * j + 1], t[7 + j], q, q2);
+#pragma unroll
+  for (int j = 0; j < 4; j++)
+#pragma unroll
+    for (int e = 0; e < 2; e++) gs_bfly<FAST>(v[4 * j + e], v[4 * j + e + 2], t[3 + j], q, q2);
+#pragma unroll
+  for (int j = 0; j < 2; j++)
+#pragma unroll
+    for (int e = 0; e < 4; e++) gs_bfly<FAST>(v[8 * j + e], v[8 * j + e + 4], t[1 + j], q, q2);
+#pragma unroll
+  for (int e = 0; e < 8; e++) {
+    uint32_t x = v[e], y = v[e + 8], c = q2;
+    if constexpr (!FAST) {  // 4q exceeds 32 bits
+      x = umin32(x, x - q);
+      y = umin32(y, y - q);
+      c = q;
+    }
+    v[e] = shoup_mul(x + y, kc, q);
+    v[e + 8] = shoup_mul(x - y + c, kcw, q);
+  }
+}
+
 // word offset of column x inside a padded in-row buffer row
 CFHE_HD int pad_col(int x) { return x + 4 * (x >> 4); }
 

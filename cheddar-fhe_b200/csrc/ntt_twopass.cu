@@ -7,11 +7,16 @@
 // __syncwarp only). The inverse transform is the mirror image. Both passes are
 // plain grids of independent 128-thread CTAs: no cluster, no cross-CTA wait.
 //
-// What makes two passes cost one trip to HBM: the host launches them over
-// chunks of at most kChunkJobs limbs (48 MiB), the second pass works in place
-// on what the first just wrote, and a chunk is well below the 126 MB L2. The
-// first pass reads HBM and writes L2; the second reads and rewrites the same
-// lines in L2; they reach HBM once, when they are evicted.
+// What keeps two passes near one trip to HBM: the second pass works in place on
+// what the first just wrote, and up to about 400 limbs (100 MiB) that is still
+// in the 126 MB L2. Chunks of kChunkJobs limbs per launch pair: the passes are
+// bound by instruction issue, and the ramp and tail of more launches cost more
+// than the second trip saves (640 limbs there and back: 341 us in chunks of
+// 192, 334 in 320, 320 in one).
+// These kernels take calls of every size. Kernels that streamed tiles with bulk
+// tensor copies and kept a prime's twiddles in shared memory, once used from
+// 256 limb transforms on, took 15 to 20 % longer forwards and the same time
+// (within 2 %) backwards at all of 11 shapes from 236 to 1600 limbs.
 //
 // The per-thread arithmetic (radix-16 register phases, Shoup twiddles, lazy
 // [0,4q) butterflies for primes below 2^30) is shared with the cluster
@@ -23,7 +28,7 @@ namespace {
 
 constexpr int kTpThreads = 128;
 constexpr int kColTile = 16;   // columns per CTA in the column pass
-constexpr int kChunkJobs = 192;
+constexpr int kChunkJobs = 640;
 // CTAs an SM holds (80 and 64 registers a thread). Measured on 188 limbs:
 // 6 and 8 are the best of 5 to 10 each, or within 2 % of it.
 constexpr int kColCtas = 6, kRowCtas = 8;
@@ -143,13 +148,12 @@ __device__ __forceinline__ void inv_cols(const NttArgs &a, const Job &j, int til
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < 16; k++) get2(xbuf + col_word(hi + 16 * k, x), v[k], w[k]);
-  gs_radix16_pre<FAST>(v, t, q, q2);
-  gs_radix16_pre<FAST>(w, t, q, q2);
-  const Tw kc = a.kc[j.l];
+  const Tw kc = a.kc[j.l], kcw = a.kcw[j.l];
+  gs_radix16_last<FAST>(v, t, kc, kcw, q, q2);
+  gs_radix16_last<FAST>(w, t, kc, kcw, q, q2);
   const uint32_t half = q >> 1;
   const bool centred = a.centred != 0;
   auto finish = [&](uint32_t r) {
-    r = shoup_mul(r, kc, q);
     r = umin32(r, r - q);
     if (centred && r > half) r -= q;
     return r;

@@ -78,6 +78,7 @@ int run_modup(const Context &c, const LevelPlan &lp, uint32_t *mu,
       a.q[k] = c.q[g];
       a.src_limb[k] = a.dst_limb[k] = (uint16_t)k;
       a.kc[k] = d.conv.pre_tw[k - d.s0];
+      a.kcw[k] = d.conv.pre_w1_tw[k - d.s0];
     }
   if (int r = launch_ntt(c, a, true)) return r;
   c.mark("modup_intt");
@@ -112,7 +113,7 @@ int run_modup(const Context &c, const LevelPlan &lp, uint32_t *mu,
   a.table = c.d_tw;
   a.n_polys = 1;
   // listed prime by prime, so that the copies of a prime in different digits
-  // are neighbours and one CTA can transform them with one set of twiddles
+  // are neighbours and the caches hold one set of twiddles at a time
   int n = 0;
   for (int g : lp.full_g)
     for (const DigitPlan &d : lp.digits)
@@ -175,6 +176,7 @@ int run_moddown_intt(const Context &c, const ConvPlan &cv, uint32_t *y, const ui
     a.src_limb[k] = (uint16_t)cv.src_pos[k];
     a.dst_limb[k] = (uint16_t)k;
     a.kc[k] = cv.pre_tw[k];
+    a.kcw[k] = cv.pre_w1_tw[k];
   }
   if (int r = launch_ntt(c, a, true)) return r;
   c.mark("moddown_intt");

@@ -49,6 +49,7 @@ int finish_conv(const Context &c, ConvPlan &cv, const std::vector<int> &restored
   for (size_t k = 0; k < cv.pre.size(); k++) {
     const uint32_t q = c.q[cv.src_g[k]];
     cv.pre_tw.push_back(make_tw(mulmod(cv.pre[k] % q, rinv_mod(q), q), q));
+    cv.pre_w1_tw.push_back(make_tw(mulmod(cv.pre_tw.back().w, c.inv_w1[cv.src_g[k]], q), q));
   }
   for (size_t m = 0; m < cv.ep_pad.size(); m++) {
     const uint32_t q = c.q[cv.dst_g[m]];
@@ -101,16 +102,6 @@ int build_plans(Context &c) {
   c.use_pdl = !(pdl && std::string(pdl) == "0");
   const char *ntt_mode = getenv("CFHE_NTT");
   c.use_twopass_ntt = !(ntt_mode && std::string(ntt_mode) == "cluster");
-  // CFHE_NTT: "tiled" = always the pipelined kernels, "twopass" / "cluster" = never, otherwise by shape
-  c.ntt_policy = !ntt_mode ? 1 : std::string(ntt_mode) == "tiled" ? 2 : 0;
-  {
-    const char *chunk = getenv("CFHE_NTT_CHUNK");
-    const char *unit = getenv("CFHE_NTT_UNIT");
-    c.ntt_chunk = chunk ? atoi(chunk) : 640;
-    if (c.ntt_chunk < 1 || c.ntt_chunk > 4096) c.ntt_chunk = 640;
-    c.ntt_unit = unit ? atoi(unit) : 4;
-    if (c.ntt_unit < 1 || c.ntt_unit > 255) c.ntt_unit = 4;
-  }
   CFHE_CUDA(cudaMalloc(&c.d_error_flag, sizeof(int)));
   CFHE_CUDA(cudaMemset(c.d_error_flag, 0, sizeof(int)));
   c.nqinv.resize(c.NP);
