@@ -124,7 +124,9 @@ struct BconvTcJob {
 };
 struct BconvTcArgs {
   int n_jobs;
-  int per_unit;     // CTAs sharing the tiles of one unit (filled by the launcher)
+  int per_unit;     // CTAs sharing the tiles of one unit (filled by the launcher, as are the next three)
+  int unit_jobs;    // jobs per unit: 1, or all where they are one conversion
+  long long src_stride, dst_stride;  // words between the jobs of a unit
   int *error_flag;  // set to 1 when a completion wait timed out
   BconvTcJob jobs[kMaxBconvJobs];
 };
