@@ -774,11 +774,20 @@ int cfhe_ctpt_gemm(cfhe_context *h, uint32_t *const *y, const uint32_t *const *x
   if (n_in < 1 || n_in > 8192 || n_out < 1 || n_out > 8192 || n_limbs < 1 || n_limbs > kMaxLimbs)
     return fail("ct-pt GEMM: unsupported shape");
   Context &c = h->c;
-  // workspace: packed activations of one limb, then the two pointer tables
-  const size_t scratch = (gemm_scratch_bytes(n_in) + 255) / 256 * 256;
+  // workspace: packed activations of two limbs (one where memory is short, or
+  // where the call has no second), then the two pointer tables
+  const size_t limb = (gemm_scratch_bytes(n_in) + 255) / 256 * 256;
   const size_t tables = (size_t)(n_in + n_out) * sizeof(void *);
-  if (int r = ensure_workspace(c, (scratch + tables + 3) / 4)) return r;
+  size_t scratch = n_limbs > 1 ? 2 * limb : limb;
+  int r = ensure_workspace(c, (scratch + tables + 3) / 4);
+  if (r && n_limbs > 1) {
+    cudaGetLastError();  // the failed allocation's
+    scratch = limb;
+    r = ensure_workspace(c, (scratch + tables + 3) / 4);
+  }
+  if (r) return r;
   uint8_t *base = reinterpret_cast<uint8_t *>(c.ws);
+  uint8_t *const packed_x[2] = {base, scratch > limb ? base + limb : nullptr};
   const uint32_t **dx = reinterpret_cast<const uint32_t **>(base + scratch);
   uint32_t **dy = reinterpret_cast<uint32_t **>(base + scratch + (size_t)n_in * sizeof(void *));
   for (int k = 0; k < n_in; k++)
@@ -788,7 +797,7 @@ int cfhe_ctpt_gemm(cfhe_context *h, uint32_t *const *y, const uint32_t *const *x
   CFHE_CUDA(cudaMemcpyAsync(dx, x, (size_t)n_in * sizeof(void *), cudaMemcpyHostToDevice, c.stream));
   CFHE_CUDA(cudaMemcpyAsync(dy, y, (size_t)n_out * sizeof(void *), cudaMemcpyHostToDevice, c.stream));
   CFHE_CUDA(cudaStreamSynchronize(c.stream));  // the host tables may go away after the call
-  { int r_ = launch_ctpt_gemm(c, dy, dx, (const uint8_t *)packed, base, n_in, n_out, gidx, n_limbs); c.mark("gemm"); return r_; }
+  { int r_ = launch_ctpt_gemm(c, dy, dx, (const uint8_t *)packed, packed_x, n_in, n_out, gidx, n_limbs); c.mark("gemm"); return r_; }
 }
 
 int cfhe_sample_uniform(cfhe_context *h, uint32_t *dst, const int *gidx, int n_limbs,

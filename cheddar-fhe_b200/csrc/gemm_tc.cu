@@ -21,11 +21,12 @@
 //   below q 2^32 (at most 4 n_in terms of 255 * 255 per accumulator: n_in up
 //   to 8192), so one Montgomery reduction finishes an output word.
 //
-// Operands are packed once per call into the shared-memory operand layout
+// Operands are packed once per limb into the shared-memory operand layout
 // (K-major, 8-row x 16-byte core matrices, no swizzle), so that a pipeline
 // stage is two contiguous bulk copies:
 //   A: activations of one limb, [tile of 128 coefficients][16-byte K chunk][16][8][16]
-//      (gemm_pack_kernel, from the limb buffers of the inputs);
+//      (from the limb buffers of the inputs: the first limb by gemm_pack_kernel,
+//      every further one inside the GEMM of the limb before);
 //   B: weight byte planes of one limb, [tile of 64 outputs][K step of 64 bytes][4][32][8][16]
 //      (built on the host by cfhe_gemm_pack_weights).
 // A CTA owns one 128 x 256 accumulator tile in tensor memory (64 outputs of
@@ -67,6 +68,12 @@ struct GemmArgs {
   int n_out;                  // outputs that exist (the last tile may be padded)
   uint32_t q, nqinv;
   int *error_flag;
+  // the next limb's activations, packed by the epilogue warps while the tensor
+  // core works on this limb's; xp_next is null where there is nothing to pack
+  uint8_t *xp_next;
+  const uint32_t *const *x;
+  size_t next_off;
+  int n_in;
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
@@ -121,6 +128,22 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t *r) {
         "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr)
       : "memory");
+}
+
+// Coefficient `row` of the 128-coefficient tile m_tile, 16-byte K chunk t (four
+// inputs; zero past n_in): the words as they lie in the A operand layout.
+__device__ __forceinline__ uint4 load_chunk(const uint32_t *const *x, size_t limb_off, int n_in, int m_tile, int row,
+                                            int t) {
+  uint32_t w[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int k = 4 * t + i;
+    w[i] = k < n_in ? x[k][limb_off + (size_t)m_tile * kGmTile + row] : 0u;
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+__device__ __forceinline__ void store_chunk(uint8_t *xp, int k_chunks, int m_tile, int row, int t, uint4 w) {
+  *reinterpret_cast<uint4 *>(xp + ((size_t)m_tile * k_chunks + t) * (kGmTile * 16) + row * 16) = w;
 }
 
 __global__ void __launch_bounds__(kGmThreads, 2) gemm_tc_kernel(const __grid_constant__ GemmArgs a) {
@@ -206,6 +229,22 @@ __global__ void __launch_bounds__(kGmThreads, 2) gemm_tc_kernel(const __grid_con
                      smem_u32(accum))
                  : "memory");
   } else if (warp < 4) {
+    // ---- meanwhile: this CTA's share of the next limb's packing, a unit being
+    // one K chunk of one tile (128 threads, 2 KiB)
+    if (a.xp_next) {
+      const int k_chunks = 4 * a.k_steps, units = (int)gridDim.y * k_chunks;
+      const int cta = blockIdx.y * gridDim.x + blockIdx.x, n_cta = gridDim.x * gridDim.y;
+      const int u0 = (int)((long long)units * cta / n_cta), u1 = (int)((long long)units * (cta + 1) / n_cta);
+      for (int u = u0; u < u1; u += 4) {  // 16 loads a thread in flight
+        uint4 w[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+          if (u + i < u1) w[i] = load_chunk(a.x, a.next_off, a.n_in, (u + i) / k_chunks, tid, (u + i) % k_chunks);
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+          if (u + i < u1) store_chunk(a.xp_next, k_chunks, (u + i) / k_chunks, tid, (u + i) % k_chunks, w[i]);
+      }
+    }
     // ---- epilogue: thread = coefficient, 8 outputs (32 columns) per tensor-memory load
     const bool arrived = mbar_wait(smem_u32(accum), 0);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -246,14 +285,7 @@ __global__ void __launch_bounds__(256) gemm_pack_kernel(uint8_t *xp, const uint3
   pdl_launch_dependents();
   pdl_wait();
   const int c = blockIdx.x * 256 + threadIdx.x, t = blockIdx.y;
-  uint32_t w[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int k = 4 * t + i;
-    w[i] = k < n_in ? x[k][limb_off + c] : 0u;
-  }
-  uint8_t *tile = xp + ((size_t)(c >> 7) * k_chunks + t) * (kGmTile * 16);
-  *reinterpret_cast<uint4 *>(tile + ((c & 127) >> 3) * 128 + (c & 7) * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+  store_chunk(xp, k_chunks, c >> 7, c & 127, t, load_chunk(x, limb_off, n_in, c >> 7, c & 127, t));
 }
 
 }  // namespace
@@ -291,15 +323,15 @@ void gemm_pack_weights_limb(uint8_t *out, const uint32_t *w, int n_in, int n_out
 }
 
 // x, y: device tables of n_in / n_out polynomial pointers ([n_limbs][N] words
-// each); wp: packed weights, limb after limb; scratch: one limb of packed
-// activations (gemm_scratch_bytes).
+// each); wp: packed weights, limb after limb; scratch: two buffers for one limb
+// of packed activations each (gemm_scratch_bytes), the second may be null.
 size_t gemm_scratch_bytes(int n_in) {
   const int k_steps = (4 * n_in + kGmStepBytes - 1) / kGmStepBytes;
   return (size_t)(kN / kGmTile) * k_steps * kGmAStage;
 }
 
 int launch_ctpt_gemm(const Context &c, uint32_t *const *y, const uint32_t *const *x, const uint8_t *wp,
-                     uint8_t *scratch, int n_in, int n_out, const int *gidx, int n_limbs) {
+                     uint8_t *const *scratch, int n_in, int n_out, const int *gidx, int n_limbs) {
   static PerDeviceOnce once;
   if (int r = once.run(c.device, [] {
         CFHE_CUDA(cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGmSmem));
@@ -313,16 +345,28 @@ int launch_ctpt_gemm(const Context &c, uint32_t *const *y, const uint32_t *const
   const int k_steps = (4 * n_in + kGmStepBytes - 1) / kGmStepBytes;
   const int n_tiles = (n_out + kGmOutTile - 1) / kGmOutTile;
   const size_t w_limb = gemm_packed_weight_bytes(n_in, n_out);
+  // Packing inside the GEMM: a CTA packs 4 / n_tiles units per K step, a step
+  // takes the two CTAs of an SM about 0.4 us each and a unit about 0.3 us, so
+  // from three output tiles on the packing hides behind the products; with
+  // fewer the stand-alone kernel is the faster one. 768 x 768,
+  // 17 limbs: 9.09 -> 8.49 ms for a single call, 10.16 -> 9.87 ms back to back (at the power limit).
+  const bool overlap = n_tiles >= 3 && scratch[1];
   for (int l = 0; l < n_limbs; l++) {
     if (gidx[l] < 0 || gidx[l] >= c.NP) {
       set_error("prime index out of range");
       return -1;
     }
     const size_t limb_off = (size_t)l * kN;
-    CFHE_CUDA(launch_kernel(c.use_pdl, gemm_pack_kernel, dim3(kN / 256, 4 * k_steps), dim3(256), 0, c.stream,
-                            scratch, x, limb_off, n_in, 4 * k_steps));
+    uint8_t *const xp = overlap ? scratch[l & 1] : scratch[0];
+    if (l == 0 || !overlap)
+      CFHE_CUDA(launch_kernel(c.use_pdl, gemm_pack_kernel, dim3(kN / 256, 4 * k_steps), dim3(256), 0, c.stream,
+                              xp, x, limb_off, n_in, 4 * k_steps));
     GemmArgs a;
-    a.xp = scratch;
+    a.xp = xp;
+    a.xp_next = overlap && l + 1 < n_limbs ? scratch[(l + 1) & 1] : nullptr;
+    a.x = x;
+    a.next_off = limb_off + kN;
+    a.n_in = n_in;
     a.wp = wp + (size_t)l * w_limb;
     a.y = y;
     a.limb_off = limb_off;

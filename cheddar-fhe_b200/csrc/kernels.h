@@ -172,7 +172,7 @@ size_t gemm_packed_weight_bytes(int n_in, int n_out);  // per limb
 size_t gemm_scratch_bytes(int n_in);
 void gemm_pack_weights_limb(uint8_t *out, const uint32_t *w, int n_in, int n_out, uint32_t q);
 int launch_ctpt_gemm(const Context &c, uint32_t *const *y, const uint32_t *const *x, const uint8_t *wp,
-                     uint8_t *scratch, int n_in, int n_out, const int *gidx, int n_limbs);
+                     uint8_t *const *scratch, int n_in, int n_out, const int *gidx, int n_limbs);
 // sampling.cu: client-side sampling and encryption
 constexpr int kErrorCdfEntries = 97;
 void error_cdf_table(double sigma, uint64_t *cdf);

@@ -69,3 +69,25 @@ def test_ctpt_gemm_argument_checks(engine40, pkg):
     packed = e.gemm_pack_weights(w, g)
     with pytest.raises(pkg.CfheError):
         e.ctpt_gemm_([x], [x], packed, [0, 999])
+
+
+@pytest.mark.parametrize("n_out", [128, 129, 200])
+def test_ctpt_gemm_packing_inside_the_products(engine40, n_out):
+    """From three output tiles (129 outputs) on, a limb's activations are packed
+    inside the products of the limb before, in two alternating buffers: odd and
+    even numbers of limbs, inputs that do not fill a K step, against one limb a
+    call (which always packs by itself)."""
+    e = engine40
+    rng = np.random.default_rng(6200 + n_out)
+    for n_in, level in ((19, 2), (33, 5)):
+        g = list(e.level_limbs(level))
+        xs = [e.to_dev(rand_limbs(rng, e.primes, g, e.n)) for _ in range(n_in)]
+        w = np.stack([rng.integers(0, int(e.primes[gi]), (n_in, n_out), dtype=np.uint64).astype(np.uint32) for gi in g])
+        ys = e.empty(n_out, len(g), e.n)
+        e.ctpt_gemm_(list(ys), xs, e.gemm_pack_weights(w, g), g)
+        for l, gi in enumerate(g):
+            x1 = [x[l:l + 1].contiguous() for x in xs]
+            y1 = e.empty(n_out, 1, e.n)
+            e.ctpt_gemm_(list(y1), x1, e.gemm_pack_weights(w[l:l + 1], [gi]), [gi])
+            e.synchronize()
+            assert e.torch.equal(y1[:, 0], ys[:, l]), (n_in, l)
