@@ -20,15 +20,17 @@ static PyObject *zero;
 
 /* ---- argument conversion: 0 on success, -1 with a Python error set ---- */
 static int get_ptr(PyObject *t, void **out) {
-  if (t == Py_None) {
-    *out = NULL;
-    return 0;
-  }
   PyObject *v = PyObject_CallMethodNoArgs(t, s_data_ptr);
   if (!v) return -1;
   *out = PyLong_AsVoidPtr(v);
   Py_DECREF(v);
   return *out == NULL && PyErr_Occurred() ? -1 : 0;
+}
+
+/* an operand that an operation can do without: None is passed on as NULL */
+static int get_optional(PyObject *t, void **out) {
+  *out = NULL;
+  return t == Py_None ? 0 : get_ptr(t, out);
 }
 
 #define SMALL_LIST 64
@@ -42,13 +44,9 @@ static void free_ptrs(ptr_list *l) {
   if (l->p != l->small) PyMem_Free(l->p);
 }
 
-static int get_ptrs(PyObject *seq, ptr_list *l) {
+static int get_ptrs(PyObject *seq, int (*get)(PyObject *, void **), ptr_list *l) {
   l->p = l->small;
   l->n = 0;
-  if (seq == Py_None) {
-    l->p = NULL;
-    return 0;
-  }
   PyObject *f = PySequence_Fast(seq, "a list of tensors is expected");
   if (!f) return -1;
   const Py_ssize_t n = PySequence_Fast_GET_SIZE(f);
@@ -59,7 +57,7 @@ static int get_ptrs(PyObject *seq, ptr_list *l) {
     return -1;
   }
   for (Py_ssize_t i = 0; i < n; i++)
-    if (get_ptr(PySequence_Fast_GET_ITEM(f, i), l->p + i)) {
+    if (get(PySequence_Fast_GET_ITEM(f, i), l->p + i)) {
       free_ptrs(l);
       l->p = l->small;
       Py_DECREF(f);
@@ -213,7 +211,7 @@ static PyObject *py_binary(PyObject *self, PyObject *const *a, Py_ssize_t n) {
   long long op;
   int_list g;
   int rc;
-  if (get_ll(a[1], &op) || get_ptr(a[2], &d) || get_ptr(a[3], &x) || get_ptr(a[4], &y) || get_ints(a[5], 'i', &g))
+  if (get_ll(a[1], &op) || get_ptr(a[2], &d) || get_ptr(a[3], &x) || get_optional(a[4], &y) || get_ints(a[5], 'i', &g))
     return NULL;
   ENTER(cfhe_binary(HANDLE(a[0]), (int)op, d, x, y, g.p, g.n));
   free_ints(&g);
@@ -227,7 +225,7 @@ static PyObject *py_const_op(PyObject *self, PyObject *const *a, Py_ssize_t n) {
   long long op;
   int_list g, k;
   int rc;
-  if (get_ll(a[1], &op) || get_ptr(a[2], &d) || get_ptr(a[3], &x) || get_ptr(a[4], &y) || get_ints(a[6], 'i', &g))
+  if (get_ll(a[1], &op) || get_ptr(a[2], &d) || get_ptr(a[3], &x) || get_optional(a[4], &y) || get_ints(a[6], 'i', &g))
     return NULL;
   if (get_ints(a[5], 'I', &k)) {
     free_ints(&g);
@@ -247,12 +245,15 @@ static PyObject *py_elementwise_multi(PyObject *self, PyObject *const *a, Py_ssi
   int_list g, k;
   int rc;
   PyObject *ret = NULL;
-  if (get_ll(a[1], &wc) || get_ll(a[2], &op) || get_ptrs(a[3], &d)) return NULL;
-  if (get_ptrs(a[4], &x)) goto free_d;
-  if (get_ptrs(a[5], &y)) goto free_x;
+  if (get_ll(a[1], &wc) || get_ll(a[2], &op) || get_ptrs(a[3], get_optional, &d)) return NULL;
+  if (get_ptrs(a[4], get_optional, &x)) goto free_d;
+  if (a[5] == Py_None)
+    y.p = NULL;
+  else if (get_ptrs(a[5], get_optional, &y))
+    goto free_x;
   if (get_ints(a[6], 'I', &k)) goto free_y;
   if (get_ints(a[7], 'i', &g)) goto free_k;
-  if ((x.p && x.n < d.n) || (y.p && y.n < d.n)) {
+  if (x.n < d.n || (y.p && y.n < d.n)) {
     PyErr_SetString(PyExc_ValueError, "operand lists shorter than the destination list");
   } else {
     ENTER(cfhe_elementwise_multi(HANDLE(a[0]), wc != 0, (int)op, (int)d.n, (u32 *const *)d.p,
@@ -292,7 +293,7 @@ static PyObject *py_permute(PyObject *self, PyObject *const *a, Py_ssize_t n) {
   long long galois;
   int_list g;
   int rc;
-  if (get_ptr(a[1], &d) || get_ptr(a[2], &s) || get_ptr(a[3], &add) || get_ll(a[4], &galois) ||
+  if (get_ptr(a[1], &d) || get_ptr(a[2], &s) || get_optional(a[3], &add) || get_ll(a[4], &galois) ||
       get_ints(a[5], 'i', &g))
     return NULL;
   ENTER(cfhe_permute(HANDLE(a[0]), d, s, add, (u32)galois, g.p, g.n));
@@ -316,8 +317,8 @@ static PyObject *py_moddown(PyObject *self, PyObject *const *a, Py_ssize_t n) {
 /* two key lists, then f */
 #define KEYS(kb, ka)                                              \
   ptr_list kb##_l, ka##_l;                                        \
-  if (get_ptrs(kb, &kb##_l)) return NULL;                         \
-  if (get_ptrs(ka, &ka##_l)) {                                    \
+  if (get_ptrs(kb, get_ptr, &kb##_l)) return NULL;                \
+  if (get_ptrs(ka, get_ptr, &ka##_l)) {                           \
     free_ptrs(&kb##_l);                                           \
     return NULL;                                                  \
   }
@@ -332,9 +333,9 @@ static PyObject *py_keyswitch(PyObject *self, PyObject *const *a, Py_ssize_t n) 
   void *p[4];
   long long level, key_main;
   int rc;
-  for (int i = 0; i < 4; i++)
+  for (int i = 0; i < 3; i++)
     if (get_ptr(a[2 + i], p + i)) return NULL;
-  if (get_ll(a[1], &level) || get_ll(a[8], &key_main)) return NULL;
+  if (get_optional(a[5], p + 3) || get_ll(a[1], &level) || get_ll(a[8], &key_main)) return NULL;
   PyObject *kb = a[6], *ka = a[7];
   KEYS(kb, ka)
   ENTER(cfhe_keyswitch(HANDLE(a[0]), (int)level, p[0], p[1], p[2], p[3], KEY_ARGS(kb, ka), (int)key_main));
@@ -361,8 +362,10 @@ static PyObject *py_hmult(PyObject *self, PyObject *const *a, Py_ssize_t n) {
 
 /* keys of several rotations: a list of lists of digit tensors, one flat table.
  * NULL entries are written for a key that is None; digits > 0 takes that many
- * of each key, 0 takes all. part >= 0: every key is a pair of lists, take that one. */
+ * of each key, 0 takes all (and a None among them is an error). part >= 0: every key
+ * is a pair of lists, take that one. */
 static int get_key_table(PyObject *keys, Py_ssize_t digits, int part, ptr_list *l) {
+  int (*const get)(PyObject *, void **) = digits ? get_optional : get_ptr;
   l->p = l->small;
   l->n = 0;
   PyObject *f = PySequence_Fast(keys, "a list of keys is expected");
@@ -396,7 +399,7 @@ static int get_key_table(PyObject *keys, Py_ssize_t digits, int part, ptr_list *
     for (Py_ssize_t j = 0; j < cnt; j++) {
       if (!d)
         l->p[l->n + j] = NULL;
-      else if (get_ptr(PySequence_Fast_GET_ITEM(d, j), l->p + l->n + j))
+      else if (get(PySequence_Fast_GET_ITEM(d, j), l->p + l->n + j))
         goto fail;
     }
     l->n += cnt;
@@ -488,8 +491,8 @@ static PyObject *py_ctpt_gemm(PyObject *self, PyObject *const *a, Py_ssize_t n) 
   int_list g;
   int rc;
   PyObject *ret = NULL;
-  if (get_ptr(a[3], &w) || get_ptrs(a[1], &y)) return NULL;
-  if (get_ptrs(a[2], &x)) goto free_y;
+  if (get_ptr(a[3], &w) || get_ptrs(a[1], get_ptr, &y)) return NULL;
+  if (get_ptrs(a[2], get_ptr, &x)) goto free_y;
   if (get_ints(a[4], 'i', &g)) goto free_x;
   ENTER(cfhe_ctpt_gemm(HANDLE(a[0]), (u32 *const *)y.p, (const u32 *const *)x.p, w, (int)x.n, (int)y.n, g.p, g.n));
   ret = PyLong_FromLong(rc);
@@ -537,9 +540,9 @@ static PyObject *py_encrypt(PyObject *self, PyObject *const *a, Py_ssize_t n) {
   void *p[5];
   int_list g;
   int rc;
-  for (int i = 0; i < 5; i++)
+  for (int i = 0; i < 4; i++)
     if (get_ptr(a[1 + i], p + i)) return NULL;
-  if (get_ints(a[6], 'i', &g)) return NULL;
+  if (get_optional(a[5], p + 4) || get_ints(a[6], 'i', &g)) return NULL;
   ENTER(cfhe_encrypt(HANDLE(a[0]), p[0], p[1], p[2], p[3], p[4], g.p, g.n));
   free_ints(&g);
   return PyLong_FromLong(rc);
