@@ -314,12 +314,20 @@ static PyObject *py_moddown(PyObject *self, PyObject *const *a, Py_ssize_t n) {
   return PyLong_FromLong(rc);
 }
 
-/* two key lists, then f */
+/* the two digit lists of a key; the library reads beta(level) entries of each */
 #define KEYS(kb, ka)                                              \
   ptr_list kb##_l, ka##_l;                                        \
+  const int beta = cfhe_beta(HANDLE(a[0]), (int)level);           \
+  if (beta < 0) return PyLong_FromLong(beta);                     \
   if (get_ptrs(kb, get_ptr, &kb##_l)) return NULL;                \
   if (get_ptrs(ka, get_ptr, &ka##_l)) {                           \
     free_ptrs(&kb##_l);                                           \
+    return NULL;                                                  \
+  }                                                               \
+  if (kb##_l.n < beta || ka##_l.n < beta) {                       \
+    free_ptrs(&kb##_l);                                           \
+    free_ptrs(&ka##_l);                                           \
+    PyErr_SetString(PyExc_ValueError, "a key holds fewer digits than the level needs"); \
     return NULL;                                                  \
   }
 #define FREE_KEYS(kb, ka) \
@@ -360,12 +368,10 @@ static PyObject *py_hmult(PyObject *self, PyObject *const *a, Py_ssize_t n) {
   return PyLong_FromLong(rc);
 }
 
-/* keys of several rotations: a list of lists of digit tensors, one flat table.
- * NULL entries are written for a key that is None; digits > 0 takes that many
- * of each key, 0 takes all (and a None among them is an error). part >= 0: every key
- * is a pair of lists, take that one. */
+/* keys or plaintexts of a transform's steps: a list of lists of tensors, one flat
+ * table, `digits` entries of each list (NULL entries for a list that is None).
+ * part >= 0: every key is a pair of lists, take that one. */
 static int get_key_table(PyObject *keys, Py_ssize_t digits, int part, ptr_list *l) {
-  int (*const get)(PyObject *, void **) = digits ? get_optional : get_ptr;
   l->p = l->small;
   l->n = 0;
   PyObject *f = PySequence_Fast(keys, "a list of keys is expected");
@@ -373,14 +379,11 @@ static int get_key_table(PyObject *keys, Py_ssize_t digits, int part, ptr_list *
   Py_ssize_t cap = SMALL_LIST;
   for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(f); i++) {
     PyObject *k = PySequence_Fast_GET_ITEM(f, i), *own = NULL, *d = NULL;
-    Py_ssize_t cnt = digits;
+    const Py_ssize_t cnt = digits;
     if (k != Py_None) {
       if (part >= 0) k = own = PySequence_GetItem(k, part);
       if (!k || !(d = PySequence_Fast(k, "a list of tensors is expected"))) goto fail;
-      const Py_ssize_t have = PySequence_Fast_GET_SIZE(d);
-      if (digits == 0)
-        cnt = have;
-      else if (have < digits) {
+      if (PySequence_Fast_GET_SIZE(d) < digits) {
         PyErr_SetString(PyExc_ValueError, "a key holds fewer digits than the level needs");
         goto fail;
       }
@@ -399,7 +402,7 @@ static int get_key_table(PyObject *keys, Py_ssize_t digits, int part, ptr_list *
     for (Py_ssize_t j = 0; j < cnt; j++) {
       if (!d)
         l->p[l->n + j] = NULL;
-      else if (get(PySequence_Fast_GET_ITEM(d, j), l->p + l->n + j))
+      else if (get_optional(PySequence_Fast_GET_ITEM(d, j), l->p + l->n + j))
         goto fail;
     }
     l->n += cnt;
@@ -417,6 +420,50 @@ static int get_key_table(PyObject *keys, Py_ssize_t digits, int part, ptr_list *
   return 0;
 }
 
+/* Keys of n_rot rotations, none of them None: a list per rotation, of which the
+ * first `digits` tensors count, or all digits of all rotations in fewer lists.
+ * The library reads n_rot * digits entries, so no fewer may come out. */
+static int get_rotation_keys(PyObject *keys, Py_ssize_t n_rot, Py_ssize_t digits, ptr_list *l) {
+  PyObject *f = PySequence_Fast(keys, "a list of keys is expected");
+  if (!f) return -1;
+  PyObject *all = PyList_New(0);
+  int per_rotation = PySequence_Fast_GET_SIZE(f) >= n_rot, rc = all ? 0 : -1;
+  for (Py_ssize_t i = 0; !rc && i < PySequence_Fast_GET_SIZE(f); i++) {
+    PyObject *d = PySequence_List(PySequence_Fast_GET_ITEM(f, i));
+    if (!d) {
+      rc = -1;
+      break;
+    }
+    if (i < n_rot && PyList_GET_SIZE(d) < digits) per_rotation = 0;
+    rc = PyList_Append(all, d);
+    Py_DECREF(d);
+  }
+  Py_DECREF(f);
+  l->p = l->small;
+  l->n = 0;
+  const Py_ssize_t want = n_rot * digits;
+  if (!rc && want > SMALL_LIST && !(l->p = (void **)PyMem_Malloc(want * sizeof(void *)))) {
+    l->p = l->small;
+    PyErr_NoMemory();
+    rc = -1;
+  }
+  for (Py_ssize_t i = 0; !rc && i < PyList_GET_SIZE(all); i++) {
+    PyObject *d = PyList_GET_ITEM(all, i);
+    for (Py_ssize_t j = 0; !rc && j < PyList_GET_SIZE(d); j++) {
+      void *p;
+      rc = get_ptr(PyList_GET_ITEM(d, j), &p);
+      if (!rc && l->n < want && (!per_rotation || j < digits)) l->p[l->n++] = p;
+    }
+  }
+  if (!rc && l->n < want) {
+    PyErr_SetString(PyExc_ValueError, "fewer keys or digits than the rotations need");
+    rc = -1;
+  }
+  Py_XDECREF(all);
+  if (rc) free_ptrs(l);
+  return rc;
+}
+
 /* (handle, level, out, bx, ax, rots, evk_b, evk_a, key_main) */
 static PyObject *py_hoisted_rotations(PyObject *self, PyObject *const *a, Py_ssize_t n) {
   NEED(9)
@@ -426,12 +473,14 @@ static PyObject *py_hoisted_rotations(PyObject *self, PyObject *const *a, Py_ssi
   for (int i = 0; i < 3; i++)
     if (get_ptr(a[2 + i], p + i)) return NULL;
   if (get_ll(a[1], &level) || get_ll(a[8], &key_main)) return NULL;
+  const int beta = cfhe_beta(HANDLE(a[0]), (int)level);
+  if (beta < 0) return PyLong_FromLong(beta);
   int_list r;
   ptr_list kb, ka;
   PyObject *ret = NULL;
   if (get_ints(a[5], 'i', &r)) return NULL;
-  if (get_key_table(a[6], 0, -1, &kb)) goto free_r;
-  if (get_key_table(a[7], 0, -1, &ka)) goto free_kb;
+  if (get_rotation_keys(a[6], r.n, beta, &kb)) goto free_r;
+  if (get_rotation_keys(a[7], r.n, beta, &ka)) goto free_kb;
   ENTER(cfhe_hoisted_rotations(HANDLE(a[0]), (int)level, p[0], p[1], p[2], r.n, r.p, (const u32 *const *)kb.p,
                                (const u32 *const *)ka.p, (int)key_main));
   ret = PyLong_FromLong(rc);

@@ -192,3 +192,53 @@ def test_optional_entries_pass(binding):
     assert b.k.elementwise_multi(1, 0, 2, [X, X], [Tensor(0x30), Tensor(0x31)], [None, None], None, [0]) == 0
     assert b.table(1, 2) == [0x30, 0x31] and b.table(2, 2) == [0, 0]
     assert b.k.elementwise_multi(1, 0, 2, [X], [X], None, None, [0]) == 0
+
+
+@pytest.mark.parametrize("count", [1, 2, 40])
+def test_hoisted_rotation_keys(binding, count):
+    """Every rotation gets its own digits, whatever the number of rotations
+    (40 of them: more pointers than the binding keeps on the stack)."""
+    b = binding
+    kb, ka = ([digits(base + 16 * r) for r in range(count)] for base in (0x1000, 0x8000))
+    rots = list(range(1, count + 1))
+    assert b.k.hoisted_rotations(1, 1, X, X, X, rots, kb, ka, 0) == 0
+    assert b.ints() == rots
+    assert b.table(0, BETA * count) == [0x1000 + 16 * r + i for r in range(count) for i in range(BETA)]
+    assert b.table(1, BETA * count) == [0x8000 + 16 * r + i for r in range(count) for i in range(BETA)]
+    # a key with more digits than the level uses (made for a higher level) is used from its first digit on
+    assert b.k.hoisted_rotations(1, 1, X, X, X, rots, [digits(0x1000 + 16 * r, 4) for r in range(count)], ka, 0) == 0
+    assert b.table(0, BETA * count) == [0x1000 + 16 * r + i for r in range(count) for i in range(BETA)]
+    # all digits in one list
+    flat = [[t for k in kb for t in k]]
+    assert b.k.hoisted_rotations(1, 1, X, X, X, rots, flat, ka, 0) == 0
+    assert b.table(0, BETA * count) == [t.addr for t in flat[0]]
+
+
+def test_hoisted_rotations_refuse_missing_keys(binding):
+    b = binding
+    k1, k2 = digits(0x1000), digits(0x2000)
+    call = b.k.hoisted_rotations
+    b.refused(TypeError, call, 1, 1, X, X, X, [1, 2], [None, k2], [k1, k2], 0)
+    b.refused(TypeError, call, 1, 1, X, X, X, [1, 2], [k1, k2], [k1, None], 0)
+    b.refused(AttributeError, call, 1, 1, X, X, X, [1, 2], [k1, [None, k2[1]]], [k1, k2], 0)
+    b.refused(ValueError, call, 1, 1, X, X, X, [1, 2], [k1], [k1, k2], 0)
+    b.refused(ValueError, call, 1, 1, X, X, X, [1, 2], [k1, k2], [k1, k2[:1]], 0)
+    b.refused(ValueError, call, 1, 1, X, X, X, list(range(1, 41)), [k1] * 40, [k1] * 39, 0)
+
+
+def test_short_digit_lists_are_refused(binding):
+    b = binding
+    k1 = digits(0x1000)
+    for kb, ka in ((k1[:1], k1), (k1, k1[:1]), ([], k1)):
+        b.refused(ValueError, b.k.hmult, 1, 1, X, X, X, X, X, X, kb, ka, 0, 1)
+        b.refused(ValueError, b.k.keyswitch, 1, 1, X, X, X, None, kb, ka, 0)
+        b.refused(ValueError, b.k.linear_transform, 1, 1, X, X, X, X, [0, 1], [None, (kb, ka)], [0], [None],
+                  [[X, X]], 0, 1)
+    # more digits than the level uses: a key made for a higher level
+    assert b.k.hmult(1, 1, X, X, X, X, X, X, digits(0x1000, 4), digits(0x2000, 4), 0, 1) == 0
+    assert b.table(0, 2) == [0x1000, 0x1001] and b.table(1, 2) == [0x2000, 0x2001]
+    # an invalid level is the library's own error
+    before = b.value("calls")
+    assert b.k.hmult(1, 2, X, X, X, X, X, X, k1, k1, 0, 1) < 0
+    assert b.k.hoisted_rotations(1, 2, X, X, X, [1], [k1], [k1], 0) < 0
+    assert b.value("calls") == before
