@@ -1005,6 +1005,14 @@ static const LevelPlan *get_plan(cfhe_context *h, int level) {
   return lp;
 }
 
+// Every digit that the level's key product reads is there (a null one would
+// fault on the GPU).
+static bool has_digits(const LevelPlan &lp, const uint32_t *const *kb, const uint32_t *const *ka) {
+  for (const DigitPlan &d : lp.digits)
+    if (!kb[d.index] || !ka[d.index]) return false;
+  return true;
+}
+
 int cfhe_beta(const cfhe_context *h, int level) {
   if (!h) return fail("null context");
   const LevelPlan *lp = h->c.plan(level);
@@ -1097,7 +1105,7 @@ int cfhe_evk_inner(cfhe_context *h, int level, uint32_t *acc_b, uint32_t *acc_a,
   CFHE_ENTER(h);
   const LevelPlan *lp = get_plan(h, level);
   if (!lp) return -1;
-  if (!acc_b || !acc_a || !modup || !evk_b || !evk_a) return fail("null argument");
+  if (!acc_b || !acc_a || !modup || !evk_b || !evk_a || !has_digits(*lp, evk_b, evk_a)) return fail("null argument");
   return run_inner(h->c, *lp, acc_b, acc_a, modup, nullptr, c0, c1, evk_b,
                    evk_a, key_main);
 }
@@ -1109,7 +1117,7 @@ int cfhe_keyswitch(cfhe_context *h, int level, uint32_t *out_b, uint32_t *out_a,
   CFHE_ENTER(h);
   const LevelPlan *lp = get_plan(h, level);
   if (!lp) return -1;
-  if (!out_b || !out_a || !d || !evk_b || !evk_a) return fail("null argument");
+  if (!out_b || !out_a || !d || !evk_b || !evk_a || !has_digits(*lp, evk_b, evk_a)) return fail("null argument");
   if (int r = ensure_workspace(h->c, keyswitch_scratch_words(*lp, 0))) return r;
   return run_keyswitch(h->c, *lp, 0, out_b, out_a, d, bx, nullptr, evk_b, evk_a,
                        key_main, h->c.ws);
@@ -1127,6 +1135,7 @@ int cfhe_hoisted_rotations(cfhe_context *h, int level, uint32_t *out,
   std::vector<uint32_t> galois(n_rot);
   for (int i = 0; i < n_rot; i++) {
     if (rot[i] == 0 || rot[i] >= h->c.n / 2) return fail("rotation distance out of range");
+    if (!has_digits(*lp, evk_b + (size_t)i * lp->beta, evk_a + (size_t)i * lp->beta)) return fail("null argument");
     galois[i] = cfhe_galois_for_rotation(h, rot[i]);
   }
   if (int r = ensure_workspace(h->c, hoisted_scratch_words(*lp))) return r;
@@ -1166,6 +1175,12 @@ int cfhe_linear_transform(cfhe_context *h, int level, int rescale, uint32_t *out
   if ((need_baby_keys && (!baby_evk_b || !baby_evk_a)) ||
       (need_giant_keys && (!giant_evk_b || !giant_evk_a)))
     return fail("null argument");
+  for (int i = 1; i < n_baby; i++)
+    if (!has_digits(*lp, baby_evk_b + (size_t)i * lp->beta, baby_evk_a + (size_t)i * lp->beta))
+      return fail("null argument");
+  for (int j = 0; j < n_giant; j++)
+    if (giant_rot[j] && !has_digits(*lp, giant_evk_b + (size_t)j * lp->beta, giant_evk_a + (size_t)j * lp->beta))
+      return fail("null argument");
   if (int r = ensure_workspace(h->c, linear_transform_scratch_words(*lp, n_baby, n_giant, rescale != 0,
                                                               !h->c.use_fused_lt)))
     return r;
@@ -1181,7 +1196,7 @@ int cfhe_hmult(cfhe_context *h, int level, uint32_t *out_b, uint32_t *out_a,
   CFHE_ENTER(h);
   const LevelPlan *lp = get_plan(h, level);
   if (!lp) return -1;
-  if (!out_b || !out_a || !b1 || !a1 || !b2 || !a2 || !evk_b || !evk_a)
+  if (!out_b || !out_a || !b1 || !a1 || !b2 || !a2 || !evk_b || !evk_a || !has_digits(*lp, evk_b, evk_a))
     return fail("null argument");
   const int type = rescale ? 2 : 0;
   if (rescale && !lp->has_rescale) return fail("level cannot be rescaled");

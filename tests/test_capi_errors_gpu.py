@@ -87,3 +87,35 @@ def test_allocator_merges_free_neighbours(engine40):
     e._check(e.L.cfhe_free(e.h, big))
     with pytest.raises(Exception, match="not returned"):
         e._check(e.L.cfhe_free(e.h, big))  # double free is refused
+
+
+@pytest.mark.parametrize("level", [1, 28])
+def test_null_key_digits_are_refused(pkg, engine40, level):
+    """Each entry that takes a key looks at every digit that it will read; the
+    checks come before any launch."""
+    e = engine40
+    L, h, p = e.L, e.h, e._p
+    nq, beta, key_main = len(e.level_limbs(level)), e.beta(level), len(e.p["main_primes"])
+    x = e.empty(2, nq, e.n)
+    mu, acc = e.empty(beta, nq + e.alpha, e.n), e.empty(2, nq + e.alpha, e.n)
+    one, two = (C.c_int * 1)(1), (C.c_int * 2)(0, 1)
+    full = [x.data_ptr()] * (2 * beta)
+    absent = len(e.p["terminal_primes"]) - e.p["level_config"][level][1]  # leading places a digit window may cover alone
+    for gap in range(absent // e.alpha, beta):
+        short = list(full)
+        short[gap] = short[beta + gap] = None
+        good, bad = ((C.c_void_p * (2 * beta))(*k) for k in (full, short))
+        for kb, ka in ((bad, good), (good, bad)):
+            calls = [
+                L.cfhe_hmult(h, level, p(x), p(x), p(x), p(x), p(x), p(x), kb, ka, key_main, 0),
+                L.cfhe_keyswitch(h, level, p(x), p(x), p(x), None, kb, ka, key_main),
+                L.cfhe_hoisted_rotations(h, level, p(x), p(x), p(x), 1, one, kb, ka, key_main),
+                L.cfhe_evk_inner(h, level, p(acc), p(acc), p(mu), None, None, kb, ka, key_main),
+                L.cfhe_linear_transform(h, level, 0, p(x), p(x), p(x), p(x), 2, two, kb, ka, 1, (C.c_int * 1)(0),
+                                        None, None, (C.c_void_p * 2)(p(mu), p(mu)), key_main),
+                L.cfhe_linear_transform(h, level, 0, p(x), p(x), p(x), p(x), 1, (C.c_int * 1)(0), None, None, 1, one,
+                                        kb, ka, (C.c_void_p * 1)(p(mu)), key_main),
+            ]
+            assert all(rc < 0 for rc in calls), calls
+            assert b"null" in L.cfhe_last_error()
+    e.synchronize()
