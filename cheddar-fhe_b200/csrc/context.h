@@ -221,6 +221,10 @@ inline cudaError_t launch_kernel(bool pdl, void (*kernel)(KArgs...), dim3 grid, 
 }
 #endif
 
+// polynomials at p, p + stride, ... all start at a multiple of `words` words
+inline bool ntt_aligned(const void *p, long long stride, int n_polys, int words) {
+  return (uintptr_t)p % (4u * words) == 0 && (n_polys <= 1 || stride % words == 0);
+}
 int launch_ntt(const Context &ctx, const NttArgs &args, bool inverse);
 int launch_ntt_twopass(const Context &ctx, const NttArgs &args, bool inverse);
 

@@ -184,7 +184,17 @@ __global__ void __cluster_dims__(kClusterSize, 1, 1)
 
 }  // namespace
 
+// The row passes move 128 bits a thread: a forward transform's destination (and
+// the operand of its epilogue) and an inverse transform's source lie on 16-byte
+// boundaries. The other side may start at any word.
 int launch_ntt(const Context &ctx, const NttArgs &args, bool inverse) {
+  if (args.n_limbs <= 0 || args.n_polys <= 0) return 0;
+  if (!(inverse ? ntt_aligned(args.src, args.src_poly_stride, args.n_polys, 4)
+                : ntt_aligned(args.dst, args.dst_poly_stride, args.n_polys, 4) &&
+                      (!args.ep_mode || ntt_aligned(args.ep_src, args.ep_poly_stride, args.n_polys, 4)))) {
+    set_error("ntt: a forward destination or an inverse source is not 16-byte aligned");
+    return -1;
+  }
   if (ctx.use_twopass_ntt) return launch_ntt_twopass(ctx, args, inverse);
   static PerDeviceOnce once;
   if (int r = once.run(ctx.device, [] {

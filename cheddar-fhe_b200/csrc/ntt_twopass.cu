@@ -82,17 +82,31 @@ __device__ __forceinline__ void ld_row_tw(const uint4 *t, Tw *out) {
 // access to memory moves 64 bits. (One column a thread: the 16 broadcast loads
 // of twiddles per 16 words kept the load pipe as busy as the butterflies keep
 // the multiplier; 62 cycles a word and warp against 54.)
+// NARROW: word by word, for a forward source or an inverse destination that
+// lies at an odd word (launch_ntt).
+template <bool NARROW = false>
 __device__ __forceinline__ void put2(uint32_t *p, uint32_t a, uint32_t b) {
-  *reinterpret_cast<uint2 *>(p) = make_uint2(a, b);
+  if constexpr (NARROW) {
+    p[0] = a;
+    p[1] = b;
+  } else {
+    *reinterpret_cast<uint2 *>(p) = make_uint2(a, b);
+  }
 }
+template <bool NARROW = false>
 __device__ __forceinline__ void get2(const uint32_t *p, uint32_t &a, uint32_t &b) {
-  const uint2 w = *reinterpret_cast<const uint2 *>(p);
-  a = w.x;
-  b = w.y;
+  if constexpr (NARROW) {
+    a = p[0];
+    b = p[1];
+  } else {
+    const uint2 w = *reinterpret_cast<const uint2 *>(p);
+    a = w.x;
+    b = w.y;
+  }
 }
 
 // ---- forward, pass 1: stages 1-8 (rows paired), src -> dst, values lazy ----
-template <bool FAST>
+template <bool FAST, bool NARROW>
 __device__ __forceinline__ void fwd_cols(const NttArgs &a, const Job &j, int tile, int tid,
                                          uint32_t *xbuf) {
   const uint32_t q = j.q, q2 = 2 * q;
@@ -103,7 +117,7 @@ __device__ __forceinline__ void fwd_cols(const NttArgs &a, const Job &j, int til
   ld_tw16(j.tw, 1, t);  // the tables are never written by a kernel: fetched before the wait
   pdl_wait();
 #pragma unroll
-  for (int k = 0; k < 16; k++) get2(s + k * 16 * kRowWords, v[k], w[k]);
+  for (int k = 0; k < 16; k++) get2<NARROW>(s + k * 16 * kRowWords, v[k], w[k]);
   if (a.premul) {
     const Tw kc = a.kc[j.l];
 #pragma unroll
@@ -128,7 +142,7 @@ __device__ __forceinline__ void fwd_cols(const NttArgs &a, const Job &j, int til
 }
 
 // ---- inverse, pass 2: strides 1..128 rows, per-limb constant, in place ----
-template <bool FAST>
+template <bool FAST, bool NARROW>
 __device__ __forceinline__ void inv_cols(const NttArgs &a, const Job &j, int tile, int tid,
                                          uint32_t *xbuf) {
   const uint32_t q = j.q, q2 = 2 * q;
@@ -139,7 +153,7 @@ __device__ __forceinline__ void inv_cols(const NttArgs &a, const Job &j, int til
   ld_tw16(j.tw, 16 + hi, t);
   pdl_wait();
 #pragma unroll
-  for (int k = 0; k < 16; k++) get2(base + (16 * hi + k) * kRowWords, v[k], w[k]);
+  for (int k = 0; k < 16; k++) get2<NARROW>(base + (16 * hi + k) * kRowWords, v[k], w[k]);
   gs_radix16_pre<FAST>(v, t, q, q2);
   gs_radix16_pre<FAST>(w, t, q, q2);
   ld_tw16(j.tw, 1, t);  // in flight across the transposition
@@ -159,7 +173,7 @@ __device__ __forceinline__ void inv_cols(const NttArgs &a, const Job &j, int til
     return r;
   };
 #pragma unroll
-  for (int k = 0; k < 16; k++) put2(base + (hi + 16 * k) * kRowWords, finish(v[k]), finish(w[k]));
+  for (int k = 0; k < 16; k++) put2<NARROW>(base + (hi + 16 * k) * kRowWords, finish(v[k]), finish(w[k]));
 }
 
 // A warp owns two rows and exchanges through its own piece of shared memory: no
@@ -313,7 +327,7 @@ __device__ __forceinline__ void inv_rows(const NttArgs &, const Job &j, int pair
 // Measured, 188 limbs of 47 primes in place: both passes 50.2 -> 40.8 us
 // forward, 55.1 -> 45.7 us inverse (256-thread CTAs, one column a thread, row
 // pass stored as the butterflies leave it); the butterflies alone take 28 us.
-template <bool INV, int PASS>
+template <bool INV, int PASS, bool NARROW>
 __global__ void __launch_bounds__(kTpThreads, PASS == 0 ? kColCtas : kRowCtas)
     ntt_twopass_kernel(const __grid_constant__ NttArgs a, const uint4 *row_table, int job0) {
   __shared__ __align__(16) uint32_t xbuf[PASS == 0 ? kColBufWords : kRowBufWordsCta];
@@ -325,9 +339,9 @@ __global__ void __launch_bounds__(kTpThreads, PASS == 0 ? kColCtas : kRowCtas)
     const int part = blockIdx.x % kTiles;
     const bool fast = j.q < (1u << 30);
     if constexpr (!INV) {
-      if (fast) fwd_cols<true>(a, j, part, tid, xbuf); else fwd_cols<false>(a, j, part, tid, xbuf);
+      if (fast) fwd_cols<true, NARROW>(a, j, part, tid, xbuf); else fwd_cols<false, NARROW>(a, j, part, tid, xbuf);
     } else {
-      if (fast) inv_cols<true>(a, j, part, tid, xbuf); else inv_cols<false>(a, j, part, tid, xbuf);
+      if (fast) inv_cols<true, NARROW>(a, j, part, tid, xbuf); else inv_cols<false, NARROW>(a, j, part, tid, xbuf);
     }
   } else {
     constexpr int kWarps = kTpThreads / 32, kCtas = kRowWords / 2 / kWarps;
@@ -348,7 +362,12 @@ __global__ void __launch_bounds__(kTpThreads, PASS == 0 ? kColCtas : kRowCtas)
 template <bool INV, int PASS>
 cudaError_t launch_pass(const Context &ctx, const NttArgs &args, int job0, int cnt) {
   const int grid = PASS == 0 ? cnt * (kRowWords / kColTile) : cnt * (kRowWords / 2) / (kTpThreads / 32);
-  return launch_kernel(ctx.use_pdl, ntt_twopass_kernel<INV, PASS>, dim3(grid), dim3(kTpThreads), 0, ctx.stream, args,
+  auto kernel = ntt_twopass_kernel<INV, PASS, false>;
+  // the side of the column pass that does not meet the row pass
+  if (PASS == 0 && !ntt_aligned(INV ? args.dst : args.src, INV ? args.dst_poly_stride : args.src_poly_stride,
+                                args.n_polys, 2))
+    kernel = ntt_twopass_kernel<INV, PASS, PASS == 0>;
+  return launch_kernel(ctx.use_pdl, kernel, dim3(grid), dim3(kTpThreads), 0, ctx.stream, args,
                        INV ? ctx.d_row_itw : ctx.d_row_tw, job0);
 }
 

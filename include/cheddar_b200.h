@@ -94,7 +94,8 @@ CFHE_API int cfhe_copy_d2h(cfhe_context *ctx, void *dst, const void *src, size_t
 /* Batched forward NTT of n_polys polynomials with the same limb list.
  * NTTHandler<word>::NTT (src/core/NTT.cu:606-671); mont_conv multiplies the
  * input by 2^32 mod q first (the reference's montgomery_conversion). Strides
- * are in words between consecutive polynomials. dst may equal src. */
+ * are in words between consecutive polynomials. dst may equal src; dst lies on a
+ * 16-byte boundary in every polynomial, src may start at any word. */
 CFHE_API int cfhe_ntt(cfhe_context *ctx, uint32_t *dst, const uint32_t *src,
              const int *gidx, int n_limbs, int n_polys,
              long long dst_poly_stride, long long src_poly_stride,

@@ -67,3 +67,46 @@ def test_bad_arguments_fail_loudly(engine40, pkg):
     a = engine40.empty(1, engine40.n)
     with pytest.raises(pkg.CfheError):
         engine40.ntt_(a, a, [engine40.num_primes])
+
+
+def view_at(e, words, polys, limbs, offset, extra):
+    """A [polys, limbs, N] view `offset` words into a buffer on a 16-byte
+    boundary, polynomials limbs * N + extra words apart."""
+    stride = limbs * e.n + extra
+    buf = e.torch.empty(offset + polys * stride, dtype=e.torch.int32, device="cuda:0")
+    v = buf.as_strided((polys, limbs, e.n), (stride, e.n, 1), offset)
+    v.copy_(words)
+    return v
+
+
+@pytest.mark.parametrize("offset,extra", [(1, 0), (2, 0), (3, 1), (0, 1), (4, 2), (0, 7)])
+def test_sides_that_may_start_at_any_word(engine40, offset, extra):
+    """The source of a forward and the destination of an inverse transform, off
+    the 8- and 16-byte boundaries by offset or by stride."""
+    e = engine40
+    rng = np.random.default_rng(15)
+    g = [0, 20, 50]  # an auxiliary prime above 2^30 among them
+    a = e.to_dev(rand_poly(rng, e.primes, g, e.n, polys=3))
+    src = view_at(e, a, 3, len(g), offset, extra)
+    want, got = e.torch.empty_like(a), e.torch.empty_like(a)
+    e.ntt_(want, a, g)
+    e.ntt_(got, src, g)
+    assert e.torch.equal(got, want) and e.torch.equal(src, a)
+    for cen in (False, True):
+        e.intt_(want, got, g, centred=cen)
+        dst = view_at(e, e.torch.zeros_like(a), 3, len(g), offset, extra)
+        e.intt_(dst, got, g, centred=cen)
+        assert e.torch.equal(dst, want)
+
+
+def test_sides_that_need_a_boundary_are_refused(engine40, pkg):
+    """Refused before any launch: the row passes' side off its 16-byte boundary."""
+    e = engine40
+    g = [0, 20]
+    a = e.torch.zeros((2, 2, e.n), dtype=e.torch.int32, device="cuda:0")
+    for offset, extra in ((1, 0), (2, 0), (0, 2)):
+        off = view_at(e, a, 2, 2, offset, extra)
+        with pytest.raises(pkg.CfheError, match="aligned"):
+            e.ntt_(off, a, g)
+        with pytest.raises(pkg.CfheError, match="aligned"):
+            e.intt_(a, off, g)
