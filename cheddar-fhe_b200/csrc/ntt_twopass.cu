@@ -127,6 +127,7 @@ __device__ __forceinline__ void fwd_cols(const NttArgs &a, const Job &j, int til
     }
   }
   ct_radix16_pre<FAST>(v, t, q, q2);
+  pdl_launch_dependents();
   ct_radix16_pre<FAST>(w, t, q, q2);
   ld_tw16(j.tw, 16 + hi, t);  // in flight across the transposition
 #pragma unroll
@@ -155,6 +156,7 @@ __device__ __forceinline__ void inv_cols(const NttArgs &a, const Job &j, int til
 #pragma unroll
   for (int k = 0; k < 16; k++) get2<NARROW>(base + (16 * hi + k) * kRowWords, v[k], w[k]);
   gs_radix16_pre<FAST>(v, t, q, q2);
+  pdl_launch_dependents();
   gs_radix16_pre<FAST>(w, t, q, q2);
   ld_tw16(j.tw, 1, t);  // in flight across the transposition
 #pragma unroll
@@ -225,6 +227,7 @@ __device__ __forceinline__ void fwd_rows(const NttArgs &a, const Job &j, int pai
 #pragma unroll
   for (int k = 0; k < 16; k++) v[k] = s[16 * k];
   ct_radix16_pre<FAST>(v, t, q, q2);
+  pdl_launch_dependents();
   ld_row_tw(j.row_tw + R * 128 + g, t);  // in flight across the exchange
 #pragma unroll
   for (int k = 0; k < 16; k++) buf[pos.strided[(k >> 1) & 3] + 16 * k] = v[k];
@@ -308,6 +311,7 @@ __device__ __forceinline__ void inv_rows(const NttArgs &, const Job &j, int pair
 #pragma unroll
   for (int i = 0; i < 4; i++) lds4(buf + pos.block[i], v + 4 * i);
   gs_radix16_pre<FAST>(v, t, q, q2);
+  pdl_launch_dependents();
   ld_tw16(j.tw, 256 + R, t);  // in flight across the exchange
 #pragma unroll
   for (int i = 0; i < 4; i++) sts4(buf + pos.block[i], v + 4 * i);
@@ -320,6 +324,16 @@ __device__ __forceinline__ void inv_rows(const NttArgs &, const Job &j, int pair
   for (int k = 0; k < 16; k++) o[16 * k] = v[k];
 }
 
+// Every pass fetches its first twiddles, waits for the kernel before it
+// (pdl_wait), and lets the next kernel's CTAs in when its own words have arrived
+// and gone through the first butterflies. Let in at the top of the kernel, CTAs
+// of several kernels ahead occupy the SMs while nothing of theirs can run, and
+// calls of few limbs take as long as without early launches: 12 limbs 11.4 us
+// forward and 12.3 inverse against 7.2 and 7.9 (9 limbs 10.5 and 6.7 forward, 23
+// limbs 12.0 and 9.6), HMult at level 1 56.0 against 52.8 us, at level 7 75.0
+// against 71.7 (GPU time, calls queued up). From 40 limbs on both are within
+// 2 %. Right after the wait is as good up to 20 limbs, but 11.6 us at 23; before
+// the first butterflies costs large inverse calls 3 to 4 %.
 // PASS 0: column pass, a CTA per tile; PASS 1: row pass, a warp per two rows.
 // Forward runs 0 then 1; inverse 1 then 0. One tile per CTA: a grid that fills
 // the GPU once and walks the tiles was 3 to 12 % slower (the SMs do not progress
@@ -331,7 +345,6 @@ template <bool INV, int PASS, bool NARROW>
 __global__ void __launch_bounds__(kTpThreads, PASS == 0 ? kColCtas : kRowCtas)
     ntt_twopass_kernel(const __grid_constant__ NttArgs a, const uint4 *row_table, int job0) {
   __shared__ __align__(16) uint32_t xbuf[PASS == 0 ? kColBufWords : kRowBufWordsCta];
-  pdl_launch_dependents();  // each pass calls pdl_wait() after its first twiddle fetch
   const int tid = threadIdx.x;
   if constexpr (PASS == 0) {
     constexpr int kTiles = kRowWords / kColTile;
