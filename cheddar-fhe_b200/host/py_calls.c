@@ -68,6 +68,29 @@ static int get_ptrs(PyObject *seq, int (*get)(PyObject *, void **), ptr_list *l)
   return 0;
 }
 
+/* operands of `count` destinations: a shorter list ends in NULLs */
+static int get_operands(PyObject *seq, Py_ssize_t count, ptr_list *l) {
+  if (get_ptrs(seq, get_optional, l)) return -1;
+  if (l->n > count) {
+    PyErr_SetString(PyExc_IndexError, "more operands than destinations");
+    free_ptrs(l);
+    return -1;
+  }
+  if (count > SMALL_LIST && l->n < count) {
+    void **longer = (void **)PyMem_Malloc(count * sizeof(void *));
+    if (!longer) {
+      free_ptrs(l);
+      PyErr_NoMemory();
+      return -1;
+    }
+    for (Py_ssize_t i = 0; i < l->n; i++) longer[i] = l->p[i];
+    free_ptrs(l);
+    l->p = longer;
+  }
+  while (l->n < count) l->p[l->n++] = NULL;
+  return 0;
+}
+
 /* 32-bit integers: a contiguous array of that type is used where it lies,
  * anything else goes through numpy. */
 typedef struct {
@@ -246,20 +269,16 @@ static PyObject *py_elementwise_multi(PyObject *self, PyObject *const *a, Py_ssi
   int rc;
   PyObject *ret = NULL;
   if (get_ll(a[1], &wc) || get_ll(a[2], &op) || get_ptrs(a[3], get_optional, &d)) return NULL;
-  if (get_ptrs(a[4], get_optional, &x)) goto free_d;
+  if (get_operands(a[4], d.n, &x)) goto free_d;
   if (a[5] == Py_None)
     y.p = NULL;
-  else if (get_ptrs(a[5], get_optional, &y))
+  else if (get_operands(a[5], d.n, &y))
     goto free_x;
   if (get_ints(a[6], 'I', &k)) goto free_y;
   if (get_ints(a[7], 'i', &g)) goto free_k;
-  if (x.n < d.n || (y.p && y.n < d.n)) {
-    PyErr_SetString(PyExc_ValueError, "operand lists shorter than the destination list");
-  } else {
-    ENTER(cfhe_elementwise_multi(HANDLE(a[0]), wc != 0, (int)op, (int)d.n, (u32 *const *)d.p,
-                                 (const u32 *const *)x.p, (const u32 *const *)y.p, k.p, g.p, g.n));
-    ret = PyLong_FromLong(rc);
-  }
+  ENTER(cfhe_elementwise_multi(HANDLE(a[0]), wc != 0, (int)op, (int)d.n, (u32 *const *)d.p,
+                               (const u32 *const *)x.p, (const u32 *const *)y.p, k.p, g.p, g.n));
+  ret = PyLong_FromLong(rc);
   free_ints(&g);
 free_k:
   free_ints(&k);

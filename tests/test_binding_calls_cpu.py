@@ -242,3 +242,18 @@ def test_short_digit_lists_are_refused(binding):
     assert b.k.hmult(1, 2, X, X, X, X, X, X, k1, k1, 0, 1) < 0
     assert b.k.hoisted_rotations(1, 2, X, X, X, [1], [k1], [k1], 0) < 0
     assert b.value("calls") == before
+
+
+def test_element_wise_list_lengths(binding):
+    """As many operands as destinations count: a shorter list ends in missing
+    operands (which the library judges), a longer one is an error."""
+    b = binding
+    call = b.k.elementwise_multi
+    assert call(1, 0, 2, [X, X], [Tensor(0x30), Tensor(0x31)], [Tensor(0x40)], None, [0]) == 0
+    assert b.table(1, 2) == [0x30, 0x31] and b.table(2, 2) == [0x40, 0]
+    assert call(1, 0, 2, [X, X], [X, X], [], None, [0]) == 0 and b.table(2, 2) == [0, 0]
+    many = [Tensor(0x1000 + i) for i in range(70)]
+    assert call(1, 0, 0, many, many, many[:65], None, [0]) == 0
+    assert b.table(2, 70) == [t.addr for t in many[:65]] + [0] * 5
+    b.refused(IndexError, call, 1, 0, 0, [X], [X, X], [X], None, [0])
+    b.refused(IndexError, call, 1, 0, 0, [X], [X], [X, X], None, [0])
