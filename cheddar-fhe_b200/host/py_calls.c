@@ -118,7 +118,7 @@ static int take_buffer(PyObject *o, char fmt, int_list *l) {
   }
   l->held = 1;
   l->p = l->b.buf;
-  l->n = (int)(l->b.len / 4);
+  l->n = l->b.ndim ? (int)l->b.shape[0] : 1; /* the rows of a 2-D array, as len() counts */
   return 1;
 }
 
@@ -126,7 +126,6 @@ static int get_ints(PyObject *o, char fmt, int_list *l) {
   l->held = 0;
   l->p = NULL;
   l->n = 0;
-  if (o == Py_None) return 0;
   if (take_buffer(o, fmt, l)) return 0;
   PyObject *a = PyObject_CallOneArg(fmt == 'i' ? as_int32 : as_uint32, o);
   if (!a) return -1;
@@ -139,17 +138,28 @@ static int get_ints(PyObject *o, char fmt, int_list *l) {
   return 0;
 }
 
+/* constants that an operation can do without */
+static int get_constants(PyObject *o, int_list *l) {
+  if (o != Py_None) return get_ints(o, 'I', l);
+  l->held = 0;
+  l->p = NULL;
+  l->n = 0;
+  return 0;
+}
+
+/* an integer (no number with a fraction, even if it is 0) */
 static int get_ll(PyObject *o, long long *out) {
   *out = PyLong_AsLongLong(o);
-  if (*out == -1 && PyErr_Occurred()) {
-    PyErr_Clear();
-    PyObject *i = PyNumber_Long(o); /* numpy scalars, floats with an integral meaning, truth values */
-    if (!i) return -1;
-    *out = PyLong_AsLongLong(i);
-    Py_DECREF(i);
-    if (*out == -1 && PyErr_Occurred()) return -1;
-  }
-  return 0;
+  return *out == -1 && PyErr_Occurred() ? -1 : 0;
+}
+
+/* what int() makes of it, modulo 2^64: flags, Galois elements, limb counts */
+static int get_converted(PyObject *o, long long *out) {
+  PyObject *i = PyNumber_Long(o);
+  if (!i) return -1;
+  *out = (long long)PyLong_AsUnsignedLongLongMask(i);
+  Py_DECREF(i);
+  return *out == -1 && PyErr_Occurred() ? -1 : 0;
 }
 
 /* number of polynomials and words between them of a [limbs, N] or [polys, limbs, N] tensor */
@@ -200,7 +210,7 @@ static PyObject *py_ntt(PyObject *self, PyObject *const *a, Py_ssize_t n) {
   int_list g;
   int rc;
   if (get_ptr(a[1], &d) || get_ptr(a[2], &s) || get_shape(a[2], &polys, &ss) || get_shape(a[1], &dp, &ds) ||
-      get_ll(a[4], &mont) || get_ints(a[3], 'i', &g))
+      get_converted(a[4], &mont) || get_ints(a[3], 'i', &g))
     return NULL;
   ENTER(cfhe_ntt(HANDLE(a[0]), d, s, g.p, g.n, (int)polys, ds, ss, mont != 0));
   free_ints(&g);
@@ -215,9 +225,9 @@ static PyObject *py_intt(PyObject *self, PyObject *const *a, Py_ssize_t n) {
   int_list g, k;
   int rc;
   if (get_ptr(a[1], &d) || get_ptr(a[2], &s) || get_shape(a[2], &polys, &ss) || get_shape(a[1], &dp, &ds) ||
-      get_ll(a[5], &keep) || get_ll(a[6], &centred) || get_ints(a[3], 'i', &g))
+      get_converted(a[5], &keep) || get_converted(a[6], &centred) || get_ints(a[3], 'i', &g))
     return NULL;
-  if (get_ints(a[4], 'I', &k)) {
+  if (get_constants(a[4], &k)) {
     free_ints(&g);
     return NULL;
   }
@@ -268,13 +278,13 @@ static PyObject *py_elementwise_multi(PyObject *self, PyObject *const *a, Py_ssi
   int_list g, k;
   int rc;
   PyObject *ret = NULL;
-  if (get_ll(a[1], &wc) || get_ll(a[2], &op) || get_ptrs(a[3], get_optional, &d)) return NULL;
+  if (get_converted(a[1], &wc) || get_converted(a[2], &op) || get_ptrs(a[3], get_optional, &d)) return NULL;
   if (get_operands(a[4], d.n, &x)) goto free_d;
   if (a[5] == Py_None)
     y.p = NULL;
   else if (get_operands(a[5], d.n, &y))
     goto free_x;
-  if (get_ints(a[6], 'I', &k)) goto free_y;
+  if (get_constants(a[6], &k)) goto free_y;
   if (get_ints(a[7], 'i', &g)) goto free_k;
   ENTER(cfhe_elementwise_multi(HANDLE(a[0]), wc != 0, (int)op, (int)d.n, (u32 *const *)d.p,
                                (const u32 *const *)x.p, (const u32 *const *)y.p, k.p, g.p, g.n));
@@ -312,7 +322,7 @@ static PyObject *py_permute(PyObject *self, PyObject *const *a, Py_ssize_t n) {
   long long galois;
   int_list g;
   int rc;
-  if (get_ptr(a[1], &d) || get_ptr(a[2], &s) || get_optional(a[3], &add) || get_ll(a[4], &galois) ||
+  if (get_ptr(a[1], &d) || get_ptr(a[2], &s) || get_optional(a[3], &add) || get_converted(a[4], &galois) ||
       get_ints(a[5], 'i', &g))
     return NULL;
   ENTER(cfhe_permute(HANDLE(a[0]), d, s, add, (u32)galois, g.p, g.n));
@@ -362,7 +372,7 @@ static PyObject *py_keyswitch(PyObject *self, PyObject *const *a, Py_ssize_t n) 
   int rc;
   for (int i = 0; i < 3; i++)
     if (get_ptr(a[2 + i], p + i)) return NULL;
-  if (get_optional(a[5], p + 3) || get_ll(a[1], &level) || get_ll(a[8], &key_main)) return NULL;
+  if (get_optional(a[5], p + 3) || get_ll(a[1], &level) || get_converted(a[8], &key_main)) return NULL;
   PyObject *kb = a[6], *ka = a[7];
   KEYS(kb, ka)
   ENTER(cfhe_keyswitch(HANDLE(a[0]), (int)level, p[0], p[1], p[2], p[3], KEY_ARGS(kb, ka), (int)key_main));
@@ -378,7 +388,7 @@ static PyObject *py_hmult(PyObject *self, PyObject *const *a, Py_ssize_t n) {
   int rc;
   for (int i = 0; i < 6; i++)
     if (get_ptr(a[2 + i], p + i)) return NULL;
-  if (get_ll(a[1], &level) || get_ll(a[10], &key_main) || get_ll(a[11], &rescale)) return NULL;
+  if (get_ll(a[1], &level) || get_converted(a[10], &key_main) || get_converted(a[11], &rescale)) return NULL;
   PyObject *kb = a[8], *ka = a[9];
   KEYS(kb, ka)
   ENTER(cfhe_hmult(HANDLE(a[0]), (int)level, p[0], p[1], p[2], p[3], p[4], p[5], KEY_ARGS(kb, ka), (int)key_main,
@@ -388,8 +398,8 @@ static PyObject *py_hmult(PyObject *self, PyObject *const *a, Py_ssize_t n) {
 }
 
 /* keys or plaintexts of a transform's steps: a list of lists of tensors, one flat
- * table, `digits` entries of each list (NULL entries for a list that is None).
- * part >= 0: every key is a pair of lists, take that one. */
+ * table, `digits` entries of each list. part >= 0: every key is a pair of lists,
+ * take that one, and a key that is None has NULL entries. */
 static int get_key_table(PyObject *keys, Py_ssize_t digits, int part, ptr_list *l) {
   l->p = l->small;
   l->n = 0;
@@ -399,7 +409,7 @@ static int get_key_table(PyObject *keys, Py_ssize_t digits, int part, ptr_list *
   for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(f); i++) {
     PyObject *k = PySequence_Fast_GET_ITEM(f, i), *own = NULL, *d = NULL;
     const Py_ssize_t cnt = digits;
-    if (k != Py_None) {
+    if (k != Py_None || part < 0) {
       if (part >= 0) k = own = PySequence_GetItem(k, part);
       if (!k || !(d = PySequence_Fast(k, "a list of tensors is expected"))) goto fail;
       if (PySequence_Fast_GET_SIZE(d) < digits) {
@@ -491,7 +501,7 @@ static PyObject *py_hoisted_rotations(PyObject *self, PyObject *const *a, Py_ssi
   int rc;
   for (int i = 0; i < 3; i++)
     if (get_ptr(a[2 + i], p + i)) return NULL;
-  if (get_ll(a[1], &level) || get_ll(a[8], &key_main)) return NULL;
+  if (get_ll(a[1], &level) || get_converted(a[8], &key_main)) return NULL;
   const int beta = cfhe_beta(HANDLE(a[0]), (int)level);
   if (beta < 0) return PyLong_FromLong(beta);
   int_list r;
@@ -519,7 +529,7 @@ static PyObject *py_linear_transform(PyObject *self, PyObject *const *a, Py_ssiz
   int rc;
   for (int i = 0; i < 4; i++)
     if (get_ptr(a[2 + i], p + i)) return NULL;
-  if (get_ll(a[1], &level) || get_ll(a[11], &key_main) || get_ll(a[12], &rescale)) return NULL;
+  if (get_ll(a[1], &level) || get_converted(a[11], &key_main) || get_converted(a[12], &rescale)) return NULL;
   const int beta = cfhe_beta(HANDLE(a[0]), (int)level);
   if (beta < 0) return PyLong_FromLong(beta);
   int_list br, gr;
@@ -576,11 +586,12 @@ free_y:
 static PyObject *py_sample_uniform(PyObject *self, PyObject *const *a, Py_ssize_t n) {
   NEED(5)
   void *d;
-  long long stream;
   int_list g;
   int rc;
   const unsigned long long seed = PyLong_AsUnsignedLongLongMask(a[3]);
-  if (PyErr_Occurred() || get_ptr(a[1], &d) || get_ll(a[4], &stream) || get_ints(a[2], 'i', &g)) return NULL;
+  if (PyErr_Occurred()) return NULL;
+  const unsigned long stream = PyLong_AsUnsignedLongMask(a[4]);
+  if (PyErr_Occurred() || get_ptr(a[1], &d) || get_ints(a[2], 'i', &g)) return NULL;
   ENTER(cfhe_sample_uniform(HANDLE(a[0]), d, g.p, g.n, seed, (unsigned)stream));
   free_ints(&g);
   return PyLong_FromLong(rc);
@@ -590,13 +601,14 @@ static PyObject *py_sample_uniform(PyObject *self, PyObject *const *a, Py_ssize_
 static PyObject *py_sample_error(PyObject *self, PyObject *const *a, Py_ssize_t n) {
   NEED(6)
   void *d;
-  long long stream;
   int_list g;
   int rc;
   const double sigma = PyFloat_AsDouble(a[3]);
   if (sigma == -1.0 && PyErr_Occurred()) return NULL;
   const unsigned long long seed = PyLong_AsUnsignedLongLongMask(a[4]);
-  if (PyErr_Occurred() || get_ptr(a[1], &d) || get_ll(a[5], &stream) || get_ints(a[2], 'i', &g)) return NULL;
+  if (PyErr_Occurred()) return NULL;
+  const unsigned long stream = PyLong_AsUnsignedLongMask(a[5]);
+  if (PyErr_Occurred() || get_ptr(a[1], &d) || get_ints(a[2], 'i', &g)) return NULL;
   ENTER(cfhe_sample_error(HANDLE(a[0]), d, g.p, g.n, sigma, seed, (unsigned)stream));
   free_ints(&g);
   return PyLong_FromLong(rc);

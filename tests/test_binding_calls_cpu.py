@@ -257,3 +257,85 @@ def test_element_wise_list_lengths(binding):
     assert b.table(2, 70) == [t.addr for t in many[:65]] + [0] * 5
     b.refused(IndexError, call, 1, 0, 0, [X], [X, X], [X], None, [0])
     b.refused(IndexError, call, 1, 0, 0, [X], [X], [X, X], None, [0])
+
+
+@pytest.mark.parametrize("gidx", [[3, 0, 7], (3, 0, 7), np.array([3, 0, 7]), np.array([3, 0, 7], dtype=np.int32),
+                                  np.array([3, 0, 7], dtype=">i4"), np.array([3, 0, 7], dtype=np.uint32),
+                                  np.array([3, 9, 0, 9, 7, 9], dtype=np.int32)[::2], range(3, 12, 4)])
+def test_index_lists(binding, gidx):
+    """Any sequence or array of integers, whatever its type, order or stride."""
+    want = list(int(i) for i in gidx)
+    assert binding.k.ntt(1, X, X, gidx, False) == 0
+    assert binding.ints() == want
+    assert binding.k.const_op(1, 0, X, X, None, gidx, gidx) == 0
+    assert binding.ints() == want
+
+
+def test_index_arrays_count_by_rows(binding):
+    """As np.ascontiguousarray and len() count: the rows of a 2-D array, one for a
+    number."""
+    assert binding.k.ntt(1, X, X, np.arange(6, dtype=np.int32).reshape(2, 3), 0) == 0
+    assert binding.ints() == [0, 1]
+    for one in (5, np.int32(5), np.array(5, dtype=np.int32)):
+        assert binding.k.ntt(1, X, X, one, 0) == 0
+        assert binding.ints() == [5]
+
+
+def test_indices_and_numbers_that_are_refused(binding):
+    b, k, key = binding, binding.k, digits(0x1000)
+    b.refused(TypeError, k.ntt, 1, X, X, None, 0)
+    b.refused(TypeError, k.const_op, 1, 0, X, X, None, None, [0])
+    b.refused(TypeError, k.hoisted_rotations, 1, 1, X, X, X, None, [key], [key], 0)
+    b.refused(TypeError, k.linear_transform, 1, 1, X, X, X, X, [0], [None], [0], [None], [None], 0, 1)
+    # a level, an operation, a stream number with a fraction
+    b.refused(TypeError, k.moddown, 1, 1.5, 0, X, X)
+    b.refused(TypeError, k.moddown, 1, 1, 0.0, X, X)
+    b.refused(TypeError, k.binary, 1, 0.0, X, X, X, [0])
+    b.refused(TypeError, k.const_op, 1, 0.5, X, X, None, [1], [0])
+    b.refused(TypeError, k.hmult, 1, 1.0, X, X, X, X, X, X, key, key, 0, 1)
+    b.refused(TypeError, k.keyswitch, 1, 1.0, X, X, X, None, key, key, 0)
+    b.refused(TypeError, k.hoisted_rotations, 1, 1.0, X, X, X, [1], [key], [key], 0)
+    b.refused(TypeError, k.linear_transform, 1, 1.0, X, X, X, X, [0], [None], [0], [None], [[X]], 0, 1)
+    b.refused(TypeError, k.sample_uniform, 1, X, [0], 1, 2.0)
+    b.refused(TypeError, k.sample_uniform, 1, X, [0], 1.0, 2)
+    b.refused(TypeError, k.sample_error, 1, X, [0], 3.2, 1, 2.0)
+
+
+def test_numbers_wrap_as_c_types(binding):
+    b = binding
+    assert b.k.sample_uniform(1, X, [0], 2 ** 64 + 5, 2 ** 32 + 7) == 0
+    assert list((C.c_longlong * 2).in_dll(b.lib, "strides")) == [5, 7]
+    assert b.k.sample_uniform(1, X, [0], 2 ** 64 - 1, 0) == 0
+    assert list((C.c_longlong * 2).in_dll(b.lib, "strides")) == [-1, 0]
+    assert b.k.permute(1, X, X, None, np.uint32(5), [0]) == 0 and b.ints() == [5]
+    assert b.k.permute(1, X, X, None, 2 ** 70 + 9, [0]) == 0 and b.ints() == [9]
+    # flags take what int() takes
+    assert b.k.ntt(1, X, X, [0], np.bool_(True)) == 0 and b.k.ntt(1, X, X, [0], 1.0) == 0
+
+
+def test_polynomials_and_strides(binding):
+    b = binding
+    assert b.k.ntt(1, Tensor(1, (5, 2, 65536), 131072), Tensor(2, (5, 2, 65536), 131073), [0, 1], 0) == 0
+    assert b.value("polys") == 5 and list((C.c_longlong * 2).in_dll(b.lib, "strides")) == [131072, 131073]
+    assert b.k.ntt(1, X, X, [0], 0) == 0 and b.value("polys") == 1
+
+
+def test_calls_from_several_threads(binding):
+    """Conversions keep nothing between calls."""
+    import threading
+    errors = []
+
+    def work(first):
+        keys = [digits(first + 16 * r) for r in range(40)]
+        for _ in range(200):
+            if binding.k.hoisted_rotations(1, 1, X, X, X, list(range(1, 41)), keys, keys, 0):
+                errors.append(first)
+            if binding.k.ctpt_gemm(1, [X] * 70, [X] * 90, X, [0, 1]):
+                errors.append(first)
+
+    threads = [threading.Thread(target=work, args=(0x10000 * (i + 1),)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
