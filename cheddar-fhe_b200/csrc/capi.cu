@@ -774,13 +774,15 @@ int cfhe_ctpt_gemm(cfhe_context *h, uint32_t *const *y, const uint32_t *const *x
   if (n_in < 1 || n_in > 8192 || n_out < 1 || n_out > 8192 || n_limbs < 1 || n_limbs > kMaxLimbs)
     return fail("ct-pt GEMM: unsupported shape");
   Context &c = h->c;
-  // workspace: packed activations of two limbs (one where memory is short, or
-  // where the call has no second), then the two pointer tables
+  // workspace: packed activations of two limbs where the next limb's are packed
+  // during the products and memory allows, otherwise of one; then the two
+  // pointer tables
   const size_t limb = (gemm_scratch_bytes(n_in) + 255) / 256 * 256;
   const size_t tables = (size_t)(n_in + n_out) * sizeof(void *);
-  size_t scratch = n_limbs > 1 ? 2 * limb : limb;
+  const bool ahead = gemm_packs_ahead(n_out, n_limbs);
+  size_t scratch = ahead ? 2 * limb : limb;
   int r = ensure_workspace(c, (scratch + tables + 3) / 4);
-  if (r && n_limbs > 1) {
+  if (r && ahead) {
     cudaGetLastError();  // the failed allocation's
     scratch = limb;
     r = ensure_workspace(c, (scratch + tables + 3) / 4);

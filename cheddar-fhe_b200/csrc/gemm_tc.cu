@@ -330,6 +330,16 @@ size_t gemm_scratch_bytes(int n_in) {
   return (size_t)(kN / kGmTile) * k_steps * kGmAStage;
 }
 
+// Whether a call packs the next limb's activations during a limb's products (and
+// wants a second buffer for that). A CTA packs 4 / n_tiles units per K step, a
+// step takes the two CTAs of an SM about 0.4 us each and a unit about 0.3 us, so
+// from three output tiles on the packing hides behind the products; with
+// fewer the stand-alone kernel is the faster one. 768 x 768,
+// 17 limbs: 9.09 -> 8.49 ms for a single call, 10.16 -> 9.87 ms back to back (at the power limit).
+bool gemm_packs_ahead(int n_out, int n_limbs) {
+  return n_limbs > 1 && (n_out + kGmOutTile - 1) / kGmOutTile >= 3;
+}
+
 int launch_ctpt_gemm(const Context &c, uint32_t *const *y, const uint32_t *const *x, const uint8_t *wp,
                      uint8_t *const *scratch, int n_in, int n_out, const int *gidx, int n_limbs) {
   static PerDeviceOnce once;
@@ -345,12 +355,7 @@ int launch_ctpt_gemm(const Context &c, uint32_t *const *y, const uint32_t *const
   const int k_steps = (4 * n_in + kGmStepBytes - 1) / kGmStepBytes;
   const int n_tiles = (n_out + kGmOutTile - 1) / kGmOutTile;
   const size_t w_limb = gemm_packed_weight_bytes(n_in, n_out);
-  // Packing inside the GEMM: a CTA packs 4 / n_tiles units per K step, a step
-  // takes the two CTAs of an SM about 0.4 us each and a unit about 0.3 us, so
-  // from three output tiles on the packing hides behind the products; with
-  // fewer the stand-alone kernel is the faster one. 768 x 768,
-  // 17 limbs: 9.09 -> 8.49 ms for a single call, 10.16 -> 9.87 ms back to back (at the power limit).
-  const bool overlap = n_tiles >= 3 && scratch[1];
+  const bool overlap = gemm_packs_ahead(n_out, n_limbs) && scratch[1];
   for (int l = 0; l < n_limbs; l++) {
     if (gidx[l] < 0 || gidx[l] >= c.NP) {
       set_error("prime index out of range");

@@ -170,6 +170,7 @@ int launch_tensor_accum(const Context &ctx, const TensorAccArgs &args);
 // gemm_tc.cu: ciphertext x plaintext RNS GEMM on the tensor cores
 size_t gemm_packed_weight_bytes(int n_in, int n_out);  // per limb
 size_t gemm_scratch_bytes(int n_in);
+bool gemm_packs_ahead(int n_out, int n_limbs);
 void gemm_pack_weights_limb(uint8_t *out, const uint32_t *w, int n_in, int n_out, uint32_t q);
 int launch_ctpt_gemm(const Context &c, uint32_t *const *y, const uint32_t *const *x, const uint8_t *wp,
                      uint8_t *const *scratch, int n_in, int n_out, const int *gidx, int n_limbs);

@@ -91,3 +91,21 @@ def test_ctpt_gemm_packing_inside_the_products(engine40, n_out):
             e.ctpt_gemm_(list(y1), x1, e.gemm_pack_weights(w[l:l + 1], [gi]), [gi])
             e.synchronize()
             assert e.torch.equal(y1[:, 0], ys[:, l]), (n_in, l)
+
+
+@pytest.mark.parametrize("n_out,buffers", [(128, 1), (129, 2)])
+def test_ctpt_gemm_workspace(pkg, params40, n_out, buffers):
+    """A second buffer of packed activations is held only by calls that pack
+    ahead (from three output tiles on)."""
+    e = pkg.Engine(params40)
+    n_in, g = 512, list(e.level_limbs(1))
+    limb = 4 * n_in * e.n  # bytes of one limb's packed activations
+    x, y = e.torch.zeros((len(g), e.n), dtype=e.torch.int32, device="cuda:0"), e.empty(n_out, len(g), e.n)
+    packed = e.gemm_pack_weights(np.zeros((len(g), n_in, n_out), dtype=np.uint32), g)
+    e.synchronize()
+    before = e.torch.cuda.mem_get_info()[0]
+    e.ctpt_gemm_(list(y), [x] * n_in, packed, g)
+    e.synchronize()
+    held = before - e.torch.cuda.mem_get_info()[0]
+    e.close()
+    assert abs(held - buffers * limb) < limb // 2, held
