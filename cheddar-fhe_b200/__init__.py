@@ -12,6 +12,8 @@ import importlib.util
 import json
 import os
 import subprocess
+import sys
+import sysconfig
 
 import numpy as np
 
@@ -19,7 +21,7 @@ from . import client  # noqa: F401  (host-side keygen / encrypt / encode)
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "lib", "libcheddar_b200.so")
-CALLS_PATH = os.path.join(_HERE, "lib", "cheddar_b200_calls.so")
+CALLS_PATH = os.path.join(_HERE, "lib", "cheddar_b200_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
 HEADER_PATH = os.path.join(os.path.dirname(_HERE), "include", "cheddar_b200.h")
 PARAM_DIR = os.path.join(_HERE, "parameters")
 
@@ -28,8 +30,9 @@ _calls = None
 
 
 def build(verbose=False):
-    """Compile every CUDA source for sm_100a into lib/libcheddar_b200.so."""
-    cmd = ["make", "-C", _HERE, "-j8"]
+    """Compile every CUDA source for sm_100a into lib/libcheddar_b200.so, and the
+    module of host/py_calls.c for this interpreter."""
+    cmd = ["make", "-C", _HERE, "-j8", f"PYTHON={sys.executable}"]
     if not verbose:
         cmd.insert(1, "-s")
     subprocess.check_call(cmd)
@@ -57,7 +60,8 @@ def calls():
         lib()
         if not os.path.exists(CALLS_PATH):
             raise RuntimeError(
-                f"{CALLS_PATH} is missing: build it with `make -C {_HERE}`; there is no fallback path")
+                f"{CALLS_PATH} is missing: build it with `make -C {_HERE} PYTHON={sys.executable}` (needs that "
+                "interpreter's headers); there is no fallback path")
         spec = importlib.util.spec_from_file_location("cheddar_b200_calls", CALLS_PATH)
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)
