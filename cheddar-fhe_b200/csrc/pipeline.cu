@@ -310,13 +310,6 @@ int run_inner(const Context &c, const LevelPlan &lp, uint32_t *acc_b,
   return run_inner_impl(c, lp, acc_b, acc_a, mu, d, c0, c1, kb, ka, key_main, 1, &none);
 }
 
-int run_inner_rot(const Context &c, const LevelPlan &lp, uint32_t *acc_b,
-                  uint32_t *acc_a, const uint32_t *mu, const uint32_t *d,
-                  const uint32_t *c0, const uint32_t *const *kb,
-                  const uint32_t *const *ka, int key_main, uint32_t galois_inv) {
-  return run_inner_impl(c, lp, acc_b, acc_a, mu, d, c0, nullptr, kb, ka, key_main, 1, &galois_inv);
-}
-
 int run_tensor(const Context &c, const LevelPlan &lp, uint32_t *d0,
                uint32_t *d1, uint32_t *d2, const uint32_t *b1,
                const uint32_t *a1, const uint32_t *b2, const uint32_t *a2) {

@@ -28,12 +28,6 @@ int run_inner(const Context &c, const LevelPlan &lp, uint32_t *acc_b,
               const uint32_t *c0, const uint32_t *c1,
               const uint32_t *const *kb, const uint32_t *const *ka,
               int key_main);
-// galois_inv != 0: the result is additionally permuted by the automorphism
-// whose inverse Galois element is galois_inv (fused into the store)
-int run_inner_rot(const Context &c, const LevelPlan &lp, uint32_t *acc_b,
-                  uint32_t *acc_a, const uint32_t *mu, const uint32_t *d,
-                  const uint32_t *c0, const uint32_t *const *kb,
-                  const uint32_t *const *ka, int key_main, uint32_t galois_inv);
 // Hoisted rotations: one ModUp of `a` shared by n_rot key switches, each fused
 // with its automorphism; out = [n_rot][2][nq][N].
 int run_hoisted_rotations(Context &c, const LevelPlan &lp, uint32_t *out,
