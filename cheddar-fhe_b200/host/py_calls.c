@@ -458,12 +458,12 @@ static int get_rotation_keys(PyObject *keys, Py_ssize_t n_rot, Py_ssize_t digits
   PyObject *all = PyList_New(0);
   int per_rotation = PySequence_Fast_GET_SIZE(f) >= n_rot, rc = all ? 0 : -1;
   for (Py_ssize_t i = 0; !rc && i < PySequence_Fast_GET_SIZE(f); i++) {
-    PyObject *d = PySequence_List(PySequence_Fast_GET_ITEM(f, i));
+    PyObject *d = PySequence_Fast(PySequence_Fast_GET_ITEM(f, i), "a list of tensors is expected");
     if (!d) {
       rc = -1;
       break;
     }
-    if (i < n_rot && PyList_GET_SIZE(d) < digits) per_rotation = 0;
+    if (i < n_rot && PySequence_Fast_GET_SIZE(d) < digits) per_rotation = 0;
     rc = PyList_Append(all, d);
     Py_DECREF(d);
   }
@@ -478,9 +478,9 @@ static int get_rotation_keys(PyObject *keys, Py_ssize_t n_rot, Py_ssize_t digits
   }
   for (Py_ssize_t i = 0; !rc && i < PyList_GET_SIZE(all); i++) {
     PyObject *d = PyList_GET_ITEM(all, i);
-    for (Py_ssize_t j = 0; !rc && j < PyList_GET_SIZE(d); j++) {
+    for (Py_ssize_t j = 0; !rc && j < PySequence_Fast_GET_SIZE(d); j++) {
       void *p;
-      rc = get_ptr(PyList_GET_ITEM(d, j), &p);
+      rc = get_ptr(PySequence_Fast_GET_ITEM(d, j), &p);
       if (!rc && l->n < want && (!per_rotation || j < digits)) l->p[l->n++] = p;
     }
   }
