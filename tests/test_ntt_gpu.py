@@ -110,3 +110,28 @@ def test_sides_that_need_a_boundary_are_refused(engine40, pkg):
             e.ntt_(off, a, g)
         with pytest.raises(pkg.CfheError, match="aligned"):
             e.intt_(a, off, g)
+
+
+def test_more_transforms_than_one_launch_covers(engine40):
+    """17 polynomials x 40 limbs: 40 transforms past the 640 of one launch pair, out
+    of place and in place, against the polynomials on both sides of the seam by
+    themselves."""
+    e = engine40
+    g = e.level_limbs(28)[:40]
+    gen = e.torch.Generator(device="cuda:0").manual_seed(17)
+    a = e.empty(17, len(g), e.n)
+    for i, gi in enumerate(g):
+        a[:, i] = e.torch.randint(0, int(e.primes[gi]), (17, e.n), dtype=e.torch.int32, device="cuda:0", generator=gen)
+    f, one = e.torch.empty_like(a), e.empty(len(g), e.n)
+    e.ntt_(f, a, g)
+    for p in (0, 15, 16):
+        e.ntt_(one, a[p], g)
+        assert e.torch.equal(f[p], one), p
+    b = a.clone()
+    e.ntt_(b, b, g)
+    assert e.torch.equal(b, f)
+    back = e.torch.empty_like(a)
+    e.intt_(back, f, g, mont_keep=True)
+    assert e.torch.equal(back, a)
+    e.intt_(b, b, g, mont_keep=True)
+    assert e.torch.equal(b, a)

@@ -406,3 +406,41 @@ def test_rotations_sharing_a_launch_equal_single_ones(engine40, level, count):
     for i, r in enumerate(rots):
         e.hoisted_rotations_(level, one, bx, ax, [r], [dk[i][0]], [dk[i][1]], 43)
         assert e.torch.equal(out[i], one[0]), r
+
+
+@pytest.fixture(scope="module")
+def engine_many_digits(pkg, params40):
+    """The prime chain of bootparam_40 with three auxiliary primes: digits of
+    three limbs, so up to eight of them at the levels used here."""
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    return pkg.Engine(dict(params40, auxiliary_primes=params40["auxiliary_primes"][:3]), device=0)
+
+
+@pytest.mark.parametrize("level,beta,active", [(8, 5, 5), (9, 6, 6), (10, 7, 6), (14, 7, 7), (15, 8, 8)])
+def test_rotations_sharing_a_launch_with_many_digits(engine_many_digits, level, beta, active):
+    """The shared launch for five to eight digits, and with a digit that the level
+    does not have, against one rotation a call."""
+    e = engine_many_digits
+    assert e.beta(level) == beta
+    nm, nt = e.p["level_config"][level]
+    assert beta - (len(e.p["terminal_primes"]) - nt) // e.alpha == active
+    gen = e.torch.Generator(device="cuda:0").manual_seed(level)
+
+    def rand(gidx, *lead):
+        out = e.empty(*lead, len(gidx), e.n)
+        for i, g in enumerate(gidx):
+            out[..., i, :] = e.torch.randint(0, int(e.primes[g]), (*lead, e.n), dtype=e.torch.int32, device="cuda:0",
+                                             generator=gen)
+        return out
+
+    g, rots = e.level_limbs(level), [3, 32767, 512, -1, 9]
+    bx, ax = rand(g), rand(g)
+    keys = rand(range(e.num_primes), len(rots), 2, beta)
+    kb, ka = ([list(k[part]) for k in keys] for part in (0, 1))
+    out, one = e.empty(len(rots), 2, len(g), e.n), e.empty(1, 2, len(g), e.n)
+    e.hoisted_rotations_(level, out, bx, ax, rots, kb, ka, 43)
+    for i, r in enumerate(rots):
+        e.hoisted_rotations_(level, one, bx, ax, [r], [kb[i]], [ka[i]], 43)
+        assert e.torch.equal(out[i], one[0]), r
