@@ -252,17 +252,17 @@ def bench_ntt(eng, pkg, torch, steps, warmup, rank, barrier):
 # algorithmic bytes of each HMult stage at a level with nq Q limbs, alpha aux
 # limbs, digit sizes ds, nd limbs after the rescale and ns limbs dropped by it
 # DRAM bytes of each HMult stage measured with ncu (warm L2) at level 28
-HMULT_STAGE_TRAFFIC = {"tensor": 60_600_000, "modup_intt": 47_800_000, "modup_bconv": 30_100_000,
-                       "modup_ntt": 69_600_000, "inner": 232_400_000, "moddown_intt": 13_200_000,
-                       "moddown_bconv": 9_200_000, "moddown_ntt": 64_000_000}
+HMULT_STAGE_TRAFFIC = {"tensor": 72_300_000, "modup_intt": 45_100_000, "modup_bconv": 30_000_000,
+                       "modup_ntt": 77_600_000, "inner": 235_700_000, "moddown_intt": 14_100_000,
+                       "moddown_bconv": 7_300_000, "moddown_ntt": 64_800_000}
 
 
 HMULT_TRAFFIC_SOURCE = ("ncu dram read+write of the stage's launches inside one HMult, warm L2 "
-                        "(--cache-control none), profiles/hmult_level28_dram_traffic.md")
+                        "(--cache-control none)")
 NTT_KERNEL_NOTE = "ntt_twopass_kernel, forward (one batch = one column-pass and one row-pass launch)"
-NTT_TRAFFIC = 706_400_000
-NTT_TRAFFIC_SOURCE = ("ncu dram read+write summed over the two launches of one forward batch, warm L2, "
-                      "profiles/ntt_twopass_kernel_batch16x40.md")
+NTT_TRAFFIC = 706_200_000
+NTT_TRAFFIC_SOURCE = ("ncu dram read+write summed over the two ntt_twopass_kernel launches of one forward batch, "
+                      "warm L2")
 
 
 def hmult_compulsory_bytes(nq, alpha, beta, nd):

@@ -191,9 +191,11 @@ const std::string &get_error();
 // attribute: a kernel may be scheduled while the previous one drains, runs
 // whatever does not depend on earlier kernels (parameter decoding, table
 // loads, tensor-memory allocation) and calls pdl_wait() before it reads or
-// writes anything an earlier kernel touches. pdl_launch_dependents() at the
-// top of a kernel lets its own successor in as soon as all of its CTAs have
-// started. Both are no-ops in a kernel launched the ordinary way.
+// writes anything an earlier kernel touches. pdl_launch_dependents() lets its
+// own successor in as soon as all of its CTAs have come to that place: the top
+// of most kernels, behind the first butterflies of a transform pass. Both are
+// no-ops in a kernel launched the ordinary way.
+
 // kernels launched by this library in this process (cfhe_kernel_launch_count)
 extern std::atomic<unsigned long long> g_kernel_launches;
 

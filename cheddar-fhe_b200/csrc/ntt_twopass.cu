@@ -15,8 +15,13 @@
 // 192, 334 in 320, 320 in one).
 // These kernels take calls of every size. Kernels that streamed tiles with bulk
 // tensor copies and kept a prime's twiddles in shared memory, once used from
-// 256 limb transforms on, took 15 to 20 % longer forwards and the same time
-// (within 2 %) backwards at all of 11 shapes from 236 to 1600 limbs.
+// 256 limb transforms on, took 15 to 19 % longer forwards and within 2 % the
+// same time backwards, but for 8 x 59 limbs, where they took 3 % less (us, both
+// timed in turn, calls queued up; forward and inverse of the removed | of these):
+// 8 x 32 limbs 71.6 66.9 | 61.1 66.0, 8 x 59 123.2 115.5 | 107.3 118.9, 12 x 40
+// 123.0 114.5 | 106.9 115.9, 16 x 40 160.6 151.3 | 139.1 150.3, 32 x 47 385 361 |
+// 328 358. Repeated for more than 0.2 s both run into the power limit (1000 W; 1765
+// MHz | 1610 MHz), which leaves 337 | 333 us for 16 x 40 there and back.
 //
 // The per-thread arithmetic (radix-16 register phases, Shoup twiddles, lazy
 // [0,4q) butterflies for primes below 2^30) is shared with the cluster
