@@ -193,7 +193,7 @@ const std::string &get_error();
 // loads, tensor-memory allocation) and calls pdl_wait() before it reads or
 // writes anything an earlier kernel touches. pdl_launch_dependents() lets its
 // own successor in as soon as all of its CTAs have come to that place: the top
-// of most kernels, behind the first butterflies of a transform pass. Both are
+// of most kernels, behind the first butterflies of a small transform. Both are
 // no-ops in a kernel launched the ordinary way.
 
 // kernels launched by this library in this process (cfhe_kernel_launch_count)

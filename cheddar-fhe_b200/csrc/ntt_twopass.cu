@@ -111,7 +111,7 @@ __device__ __forceinline__ void get2(const uint32_t *p, uint32_t &a, uint32_t &b
 }
 
 // ---- forward, pass 1: stages 1-8 (rows paired), src -> dst, values lazy ----
-template <bool FAST, bool NARROW>
+template <bool FAST, bool LATE, bool NARROW>
 __device__ __forceinline__ void fwd_cols(const NttArgs &a, const Job &j, int tile, int tid,
                                          uint32_t *xbuf) {
   const uint32_t q = j.q, q2 = 2 * q;
@@ -132,7 +132,7 @@ __device__ __forceinline__ void fwd_cols(const NttArgs &a, const Job &j, int til
     }
   }
   ct_radix16_pre<FAST>(v, t, q, q2);
-  pdl_launch_dependents();
+  if constexpr (LATE) pdl_launch_dependents();
   ct_radix16_pre<FAST>(w, t, q, q2);
   ld_tw16(j.tw, 16 + hi, t);  // in flight across the transposition
 #pragma unroll
@@ -148,7 +148,7 @@ __device__ __forceinline__ void fwd_cols(const NttArgs &a, const Job &j, int til
 }
 
 // ---- inverse, pass 2: strides 1..128 rows, per-limb constant, in place ----
-template <bool FAST, bool NARROW>
+template <bool FAST, bool LATE, bool NARROW>
 __device__ __forceinline__ void inv_cols(const NttArgs &a, const Job &j, int tile, int tid,
                                          uint32_t *xbuf) {
   const uint32_t q = j.q, q2 = 2 * q;
@@ -161,7 +161,7 @@ __device__ __forceinline__ void inv_cols(const NttArgs &a, const Job &j, int til
 #pragma unroll
   for (int k = 0; k < 16; k++) get2<NARROW>(base + (16 * hi + k) * kRowWords, v[k], w[k]);
   gs_radix16_pre<FAST>(v, t, q, q2);
-  pdl_launch_dependents();
+  if constexpr (LATE) pdl_launch_dependents();
   gs_radix16_pre<FAST>(w, t, q, q2);
   ld_tw16(j.tw, 1, t);  // in flight across the transposition
 #pragma unroll
@@ -219,7 +219,7 @@ __device__ __forceinline__ void lds4(const uint32_t *p, uint32_t *v) {
 // shared memory so that global memory sees whole lines: stored as they are
 // (128 bits a lane, 64 bytes between lanes) the pass took 72 cycles a word and
 // warp, this way 56.
-template <bool FAST>
+template <bool FAST, bool LATE>
 __device__ __forceinline__ void fwd_rows(const NttArgs &a, const Job &j, int pair, int lane, const RowPos &pos,
                                          uint32_t *buf) {
   const uint32_t q = j.q, q2 = 2 * q;
@@ -232,7 +232,7 @@ __device__ __forceinline__ void fwd_rows(const NttArgs &a, const Job &j, int pai
 #pragma unroll
   for (int k = 0; k < 16; k++) v[k] = s[16 * k];
   ct_radix16_pre<FAST>(v, t, q, q2);
-  pdl_launch_dependents();
+  if constexpr (LATE) pdl_launch_dependents();
   ld_row_tw(j.row_tw + R * 128 + g, t);  // in flight across the exchange
 #pragma unroll
   for (int k = 0; k < 16; k++) buf[pos.strided[(k >> 1) & 3] + 16 * k] = v[k];
@@ -297,7 +297,7 @@ __device__ __forceinline__ void fwd_rows(const NttArgs &a, const Job &j, int pai
 }
 
 // ---- inverse, pass 1: strides 1..128 words (inside rows), src -> dst ----
-template <bool FAST>
+template <bool FAST, bool LATE>
 __device__ __forceinline__ void inv_rows(const NttArgs &, const Job &j, int pair, int lane, const RowPos &pos,
                                          uint32_t *buf) {
   const uint32_t q = j.q, q2 = 2 * q;
@@ -316,7 +316,7 @@ __device__ __forceinline__ void inv_rows(const NttArgs &, const Job &j, int pair
 #pragma unroll
   for (int i = 0; i < 4; i++) lds4(buf + pos.block[i], v + 4 * i);
   gs_radix16_pre<FAST>(v, t, q, q2);
-  pdl_launch_dependents();
+  if constexpr (LATE) pdl_launch_dependents();
   ld_tw16(j.tw, 256 + R, t);  // in flight across the exchange
 #pragma unroll
   for (int i = 0; i < 4; i++) sts4(buf + pos.block[i], v + 4 * i);
@@ -329,16 +329,10 @@ __device__ __forceinline__ void inv_rows(const NttArgs &, const Job &j, int pair
   for (int k = 0; k < 16; k++) o[16 * k] = v[k];
 }
 
-// Every pass fetches its first twiddles, waits for the kernel before it
-// (pdl_wait), and lets the next kernel's CTAs in when its own words have arrived
-// and gone through the first butterflies. Let in at the top of the kernel, CTAs
-// of several kernels ahead occupy the SMs while nothing of theirs can run, and
-// calls of few limbs take as long as without early launches: 12 limbs 11.4 us
-// forward and 12.3 inverse against 7.2 and 7.9 (9 limbs 10.5 and 6.7 forward, 23
-// limbs 12.0 and 9.6), HMult at level 1 56.0 against 52.8 us, at level 7 75.0
-// against 71.7 (GPU time, calls queued up). From 40 limbs on both are within
-// 2 %. Right after the wait is as good up to 20 limbs, but 11.6 us at 23; before
-// the first butterflies costs large inverse calls 3 to 4 %.
+// Every pass fetches its first twiddles and waits for the kernel before it
+// (pdl_wait). LATE: it lets the next kernel's CTAs in when its own words have
+// arrived and gone through the first butterflies, otherwise at its top
+// (launch_pass holds the rule).
 // PASS 0: column pass, a CTA per tile; PASS 1: row pass, a warp per two rows.
 // Forward runs 0 then 1; inverse 1 then 0. One tile per CTA: a grid that fills
 // the GPU once and walks the tiles was 3 to 12 % slower (the SMs do not progress
@@ -346,10 +340,11 @@ __device__ __forceinline__ void inv_rows(const NttArgs &, const Job &j, int pair
 // Measured, 188 limbs of 47 primes in place: both passes 50.2 -> 40.8 us
 // forward, 55.1 -> 45.7 us inverse (256-thread CTAs, one column a thread, row
 // pass stored as the butterflies leave it); the butterflies alone take 28 us.
-template <bool INV, int PASS, bool NARROW>
+template <bool INV, int PASS, bool LATE, bool NARROW>
 __global__ void __launch_bounds__(kTpThreads, PASS == 0 ? kColCtas : kRowCtas)
     ntt_twopass_kernel(const __grid_constant__ NttArgs a, const uint4 *row_table, int job0) {
   __shared__ __align__(16) uint32_t xbuf[PASS == 0 ? kColBufWords : kRowBufWordsCta];
+  if constexpr (!LATE) pdl_launch_dependents();
   const int tid = threadIdx.x;
   if constexpr (PASS == 0) {
     constexpr int kTiles = kRowWords / kColTile;
@@ -357,9 +352,9 @@ __global__ void __launch_bounds__(kTpThreads, PASS == 0 ? kColCtas : kRowCtas)
     const int part = blockIdx.x % kTiles;
     const bool fast = j.q < (1u << 30);
     if constexpr (!INV) {
-      if (fast) fwd_cols<true, NARROW>(a, j, part, tid, xbuf); else fwd_cols<false, NARROW>(a, j, part, tid, xbuf);
+      if (fast) fwd_cols<true, LATE, NARROW>(a, j, part, tid, xbuf); else fwd_cols<false, LATE, NARROW>(a, j, part, tid, xbuf);
     } else {
-      if (fast) inv_cols<true, NARROW>(a, j, part, tid, xbuf); else inv_cols<false, NARROW>(a, j, part, tid, xbuf);
+      if (fast) inv_cols<true, LATE, NARROW>(a, j, part, tid, xbuf); else inv_cols<false, LATE, NARROW>(a, j, part, tid, xbuf);
     }
   } else {
     constexpr int kWarps = kTpThreads / 32, kCtas = kRowWords / 2 / kWarps;
@@ -370,9 +365,9 @@ __global__ void __launch_bounds__(kTpThreads, PASS == 0 ? kColCtas : kRowCtas)
     const RowPos pos(lane);
     const bool fast = j.q < (1u << 30);
     if constexpr (!INV) {
-      if (fast) fwd_rows<true>(a, j, pair, lane, pos, buf); else fwd_rows<false>(a, j, pair, lane, pos, buf);
+      if (fast) fwd_rows<true, LATE>(a, j, pair, lane, pos, buf); else fwd_rows<false, LATE>(a, j, pair, lane, pos, buf);
     } else {
-      if (fast) inv_rows<true>(a, j, pair, lane, pos, buf); else inv_rows<false>(a, j, pair, lane, pos, buf);
+      if (fast) inv_rows<true, LATE>(a, j, pair, lane, pos, buf); else inv_rows<false, LATE>(a, j, pair, lane, pos, buf);
     }
   }
 }
@@ -380,11 +375,25 @@ __global__ void __launch_bounds__(kTpThreads, PASS == 0 ? kColCtas : kRowCtas)
 template <bool INV, int PASS>
 cudaError_t launch_pass(const Context &ctx, const NttArgs &args, int job0, int cnt) {
   const int grid = PASS == 0 ? cnt * (kRowWords / kColTile) : cnt * (kRowWords / 2) / (kTpThreads / 32);
-  auto kernel = ntt_twopass_kernel<INV, PASS, false>;
+  // When the next kernel's CTAs are let in (GPU time, calls queued up, us):
+  // * Late where the row pass fits the GPU at once (37 limbs). At the top, CTAs of
+  //   several kernels ahead occupy the SMs while nothing of theirs can run, and
+  //   small calls take as long as without early launches: 12 limbs 11.1 forward and
+  //   12.2 inverse, late 7.4 and 8.1; 23 limbs 12.1 and 12.9, late 9.8 and 10.6;
+  //   HMult at level 1 56.0, late 53.0, at level 7 75.0, late 71.9. (Right after
+  //   the wait is as good up to 20 limbs, but 11.6 at 23.)
+  // * At the top above that: the last CTAs start when the others are done, and
+  //   every microsecond that they keep the next kernel out is lost: eight hoisted
+  //   rotations at level 12 281.4, late 286.3, at level 28 607.6, late 613.0.
+  // * Late again for inverse calls of more than 128 limbs (batches; the operators of
+  //   the parameter sets have at most 112): 16 x 40 limbs 149.9, late 147.8, 32
+  //   x 47 360.8, late 355.9; up to 3 x 47 both are within 1 %.
+  const bool late = cnt * (kRowWords / 2) / (kTpThreads / 32) <= ctx.num_sms * kRowCtas || (INV && cnt > 128);
+  auto kernel = late ? ntt_twopass_kernel<INV, PASS, true, false> : ntt_twopass_kernel<INV, PASS, false, false>;
   // the side of the column pass that does not meet the row pass
   if (PASS == 0 && !ntt_aligned(INV ? args.dst : args.src, INV ? args.dst_poly_stride : args.src_poly_stride,
                                 args.n_polys, 2))
-    kernel = ntt_twopass_kernel<INV, PASS, PASS == 0>;
+    kernel = ntt_twopass_kernel<INV, PASS, true, PASS == 0>;
   return launch_kernel(ctx.use_pdl, kernel, dim3(grid), dim3(kTpThreads), 0, ctx.stream, args,
                        INV ? ctx.d_row_itw : ctx.d_row_tw, job0);
 }
